@@ -83,6 +83,17 @@ __device__ __forceinline__ bool in_bulk(const MeshK &m, uint32_t c) {
          c2 < m.dims[1] - m.guard[1] && c3 < (uint32_t)m.dims[2];
 }
 
+// The same bulk test with one multiply-high for the row (a 3D grid is refused
+// at context creation, so a cell past the first plane is outside); row and
+// column of a bulk cell in c2 and c1.
+__device__ __forceinline__ bool bulk_cell(const MeshK &m, uint32_t c, int &c1, int &c2) {
+  const uint32_t q = (uint32_t)__umul64hi((unsigned long long)c, m.div0);
+  c1 = (int)(c - q * (uint32_t)m.dims[0]);
+  c2 = (int)q;
+  return q < (uint32_t)m.dims[1] && c1 >= m.guard[0] && c1 < m.dims[0] - m.guard[0] &&
+         c2 >= m.guard[1] && c2 < m.dims[1] - m.guard[1];
+}
+
 // Interpolator2D with spline_t<1> (interpolation.cuh:146-171) over the
 // reference's 3 x 3 nodes, in its summation order; st0 / st1 are the x / y
 // stagger bits.
@@ -101,7 +112,7 @@ __device__ float interp2d(const FieldArr &f, float x1, float x2, int c1, int c2,
     for (int i = 0; i <= 2; i++) {
       const int ii = i + c1 - 1;
       const float wx = cic(((float)ii + (st0 == 0 ? 0.5f : 1.0f)) - (x1 + (float)c1));
-      r += f.ptr[(size_t)jj * f.pitch + ii] * wx * wy;
+      r += __ldg(f.ptr + (size_t)jj * f.pitch + ii) * wx * wy;
     }
   }
   return r;
@@ -266,6 +277,17 @@ __device__ void produce_pair_gap(const RadK &K, const PhK &ph, size_t tid, const
   }
 }
 
+// What decides most particles from gamma alone, before the draws: the default
+// model's whole test; for the pulsar model a particle can emit only if
+// e_curv gamma^3 / rho_c > 2.1 with rho_c >= 1 (check_emit returns false for
+// smaller ones), and a rounded quotient by a number >= 1 is no larger than
+// its numerator.
+__device__ __forceinline__ bool may_emit(const RadK &K, float gamma) {
+  if (K.model == AP_RAD_DEFAULT) return gamma > K.gamma_thr;
+  if (K.model == AP_RAD_PULSAR) return K.e_curv * gamma * gamma * gamma > 2.1f;
+  return true;
+}
+
 // check_emit_photon (default :13-17; pulsar :26-53).
 __device__ bool check_emit(const RadK &K, const PtcK &p, size_t tid, uint32_t cell,
                            const float u[4]) {
@@ -278,10 +300,26 @@ __device__ bool check_emit(const RadK &K, const PtcK &p, size_t tid, uint32_t ce
   if (r > 0.6f / K.omega) return false;
   if ((double)r < 1.05) return false;
   const float theta = mpos(K.m, 1, c2, p.x2[tid]);
+  const float num = K.delta_t * gamma;
+  const float en = K.e_curv * gamma * gamma * gamma;
+  {
+    // rho_c in float (a few units of 2^-24 off the double expression rounded
+    // to float) decides all particles outside a band of 1e-4 around each
+    // threshold, without the double pow; the rest, and NaNs, take the
+    // reference's expression
+    const float c = cosf(theta), sn = sinf(theta);
+    const float t = 1.0f + 3.0f * (c * c);
+    if (sn > 1.0e-4f) {
+      const float rf = r * (t * sqrtf(t)) / (3.0f * sn * (1.0f + c * c));
+      const float rate = num / (K.l_curv * rf), eph = en / rf;
+      if (rf < 0.9999f || u[0] > rate * 1.0001f || eph < 2.1f * 0.9999f) return false;
+      if (rf > 1.0001f && u[0] < rate * 0.9999f && eph > 2.1f * 1.0001f) return true;
+    }
+  }
   const float rc = rho_c(r, theta);
   if (rc < 1.0f) return false;
-  const float rate = K.delta_t * gamma / (K.l_curv * rc);
-  const float Eph = K.e_curv * gamma * gamma * gamma / rc;
+  const float rate = num / (K.l_curv * rc);
+  const float Eph = en / rc;
   return u[0] < rate && Eph > 2.1f;
 }
 
@@ -359,29 +397,23 @@ __device__ void emit_photon(const RadK &K, const PtcK &p, size_t tid, const PhK 
   ph.cell[off] = c;
 }
 
-// check_produce_pair (default :65-68; pulsar :134-171); the pulsar checks
-// remove photons by the axis and in dense plasma.
-__device__ bool check_pair(const RadK &K, const PhK &ph, size_t tid, uint32_t cell) {
-  if (K.model == AP_RAD_DEFAULT) return ph.path[tid] <= 0.0f;
-  const int c1 = c1_of(K.m, cell), c2 = c2_of(K.m, cell);
-  const float x1 = ph.x1[tid], x2 = ph.x2[tid];
-  const float p1 = ph.p1[tid], p2 = ph.p2[tid], p3 = ph.p3[tid];
-  const float Eph = ph.E[tid];
+// check_produce_pair (default :65-68; pulsar :134-171): the pulsar test of a
+// photon whose members are loaded; `gone` is set for photons it removes, by
+// the axis and in dense plasma.
+__device__ __forceinline__ bool check_pair_pulsar(const RadK &K, float x1, float x2, float p1,
+                                                  float p2, float p3, float Eph, int c1, int c2,
+                                                  bool &gone) {
   const float theta = mpos(K.m, 1, c2, x2);
-  if (theta < K.m.delta[1] || (double)theta > kPi - (double)K.m.delta[1]) {
-    ph.cell[tid] = AP_MAX_CELL;
-    return false;
-  }
-  const float r0 = K.Rho[0].ptr[(size_t)c2 * K.Rho[0].pitch + c1];
-  const float r1 = K.Rho[1].ptr[(size_t)c2 * K.Rho[1].pitch + c1];
+  gone = true;
+  if (theta < K.m.delta[1] || (double)theta > kPi - (double)K.m.delta[1]) return false;
+  const float r0 = __ldg(K.Rho[0].ptr + (size_t)c2 * K.Rho[0].pitch + c1);
+  const float r1 = __ldg(K.Rho[1].ptr + (size_t)c2 * K.Rho[1].pitch + c1);
   const float s = fabsf(r0 + r1);
   const float rho = s < 0.0001f ? 0.0001f : s;  // max(s, 0.0001f)
   const float N = fabsf(r0) + fabsf(r1);
   const float multiplicity = N / rho;
-  if (multiplicity > 50.0f) {
-    ph.cell[tid] = AP_MAX_CELL;
-    return false;
-  }
+  if (multiplicity > 50.0f) return false;
+  gone = false;
   const float B1 = interp2d(K.B[0], x1, x2, c1, c2, 1, 0);
   const float B2 = interp2d(K.B[1], x1, x2, c1, c2, 0, 1);
   const float B3 = interp2d(K.B[2], x1, x2, c1, c2, 0, 0);
@@ -430,7 +462,8 @@ __device__ __forceinline__ void add_produced(const RadK &K, uint32_t cell, float
   const uint32_t key = on ? cell : AP_MAX_CELL;
   const unsigned peers = __match_any_sync(0xffffffffu, key);
   float sum = 0.0f;
-  for (int o = 0; o < 32; ++o) {
+  for (unsigned m = any; m != 0u; m &= m - 1u) {  // the lanes that add, in order
+    const int o = __ffs(m) - 1;
     const float v = __shfl_sync(0xffffffffu, w, o);
     if ((peers >> o) & 1u) sum += v;
   }
@@ -440,41 +473,47 @@ __device__ __forceinline__ void add_produced(const RadK &K, uint32_t cell, float
               sum);
 }
 
-// Exclusive scan of the chunk counts (one CTA of 1024 threads); the total
-// goes to offs[nchunks].
+// Exclusive scan of the chunk counts (one CTA of 1024 threads, eight
+// consecutive counts per thread and round); the total goes to offs[nchunks].
 __global__ void __launch_bounds__(1024) k_rad_scan(const uint32_t *counts, uint32_t nchunks,
                                                    uint32_t *offs) {
+  constexpr int kPer = 8;
   __shared__ uint32_t s_warp[32];
-  __shared__ uint32_t s_carry;
-  if (threadIdx.x == 0) s_carry = 0;
-  __syncthreads();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  for (uint32_t b0 = 0; b0 < nchunks; b0 += blockDim.x) {
-    const uint32_t i = b0 + threadIdx.x;
-    const uint32_t v = i < nchunks ? counts[i] : 0u;
-    uint32_t x = v;
+  uint32_t carry = 0;
+  for (uint32_t b0 = 0; b0 < nchunks; b0 += kPer * blockDim.x) {
+    const uint32_t i = b0 + threadIdx.x * kPer;
+    uint32_t v[kPer], own = 0;
+#pragma unroll
+    for (int k = 0; k < kPer; ++k) {
+      v[k] = i + k < nchunks ? counts[i + k] : 0u;
+      own += v[k];
+    }
+    uint32_t x = own;
+#pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
       const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
       if (lane >= o) x += y;
     }
     if (lane == 31) s_warp[warp] = x;
     __syncthreads();
-    if (warp == 0) {
-      uint32_t w = lane < (int)(blockDim.x >> 5) ? s_warp[lane] : 0u;
-      for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t y = __shfl_up_sync(0xffffffffu, w, o);
-        if (lane >= o) w += y;
-      }
-      s_warp[lane] = w;
+    uint32_t w = s_warp[lane];  // every warp scans the warp sums
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t y = __shfl_up_sync(0xffffffffu, w, o);
+      if (lane >= o) w += y;
     }
-    __syncthreads();
-    const uint32_t before = (warp ? s_warp[warp - 1] : 0u) + s_carry;
-    if (i < nchunks) offs[i] = before + x - v;
-    __syncthreads();
-    if (threadIdx.x == blockDim.x - 1) s_carry = before + x;
+    const uint32_t wb = __shfl_sync(0xffffffffu, w, warp > 0 ? warp - 1 : 0);
+    uint32_t run = carry + (warp > 0 ? wb : 0u) + x - own;
+#pragma unroll
+    for (int k = 0; k < kPer; ++k) {
+      if (i + k < nchunks) offs[i + k] = run;
+      run += v[k];
+    }
+    carry += __shfl_sync(0xffffffffu, w, 31);
     __syncthreads();
   }
-  if (threadIdx.x == 0) offs[nchunks] = s_carry;
+  if (threadIdx.x == 0) offs[nchunks] = carry;
 }
 
 // Rank of each of this thread's four slots (ch * 1024 + 4 t + [0, 4)) among
@@ -507,29 +546,98 @@ __device__ __forceinline__ uint32_t chunk_ranks(const uint8_t *mark, size_t numb
   return off_ch + before + x - mine;
 }
 
+// Sum over the block of each thread's count (thread 0 gets it); one barrier,
+// and one before the scratch is used again.
+__device__ __forceinline__ uint32_t block_count(uint32_t mine) {
+  __shared__ uint32_t s_w[kRadThreads / 32];
+  const uint32_t w = __reduce_add_sync(0xffffffffu, mine);
+  __syncthreads();
+  if ((threadIdx.x & 31) == 0) s_w[threadIdx.x >> 5] = w;
+  __syncthreads();
+  uint32_t sum = 0;
+  if (threadIdx.x == 0)
+#pragma unroll
+    for (int i = 0; i < kRadThreads / 32; ++i) sum += s_w[i];
+  return sum;
+}
+
+// Both marks test a few of a warp's 128 slots with long arithmetic (Philox
+// draws, transcendentals, field interpolations): the slots that need the test
+// are listed per warp first and the warp works through the list 32 at a time,
+// so its lanes are full, instead of walking all four slots of each lane with
+// the others idle. One barrier pair per chunk instead of one barrier per slot.
+struct WarpList {
+  uint8_t slot[kRadThreads / 32][32 * kRadPer];  // listed slots, k * 32 + lane
+  uint8_t hit[kRadThreads / 32][32 * kRadPer];   // the test's answer per slot
+};
+
+// Lists the slots with want[k] set and runs test(index in the store) on each;
+// bit k of the result: slot k of this lane passed.
+template <class Test>
+__device__ __forceinline__ uint32_t test_listed(WarpList &L, size_t first_of_chunk,
+                                                const bool want[kRadPer], Test &&test) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const uint32_t lt = (1u << lane) - 1u;
+  int n = 0;
+#pragma unroll
+  for (int k = 0; k < kRadPer; ++k) {
+    const uint32_t m = __ballot_sync(0xffffffffu, want[k]);
+    if (want[k]) L.slot[warp][n + __popc(m & lt)] = (uint8_t)(k * 32 + lane);
+    L.hit[warp][k * 32 + lane] = 0;
+    n += __popc(m);
+  }
+  __syncwarp();
+  for (int r = lane; r < n; r += 32) {
+    const int e = L.slot[warp][r];
+    const size_t idx = first_of_chunk + (size_t)(e >> 5) * kRadThreads + warp * 32 + (e & 31);
+    if (test(idx)) L.hit[warp][e] = 1;
+  }
+  __syncwarp();
+  uint32_t em = 0;
+#pragma unroll
+  for (int k = 0; k < kRadPer; ++k) em |= (uint32_t)L.hit[warp][k * 32 + lane] << k;
+  __syncwarp();
+  return em;
+}
+
 __global__ void __launch_bounds__(kRadThreads)
     k_rad_emit_mark(RadK K, PtcK p, const uint64_t *ids, size_t number, uint8_t *mark,
                     uint32_t *counts, uint32_t nchunks) {
+  __shared__ WarpList L;
   for (uint32_t ch = blockIdx.x; ch < nchunks; ch += gridDim.x) {
-    int cnt = 0;
-#pragma unroll 1
+    const size_t first = (size_t)ch * kRadChunk + threadIdx.x;
+    uint32_t cell[kRadPer], flag[kRadPer];
+    float gam[kRadPer];
+#pragma unroll
     for (int k = 0; k < kRadPer; ++k) {
-      const size_t idx = (size_t)ch * kRadChunk + (size_t)k * kRadThreads + threadIdx.x;
-      bool e = false;
-      uint32_t cell = AP_MAX_CELL;
-      if (idx < number) {
-        cell = p.cell[idx];
-        if (cell != AP_MAX_CELL && in_bulk(K.m, cell) && (p.flag[idx] >> 29) != 2u) {
-          float u[4];
-          uniforms(K, 1u, ids[idx], u);
-          e = check_emit(K, p, idx, cell, u);
-        }
-        mark[idx] = e ? 1 : 0;
-      }
-      if (K.produced.ptr) add_produced(K, cell, e ? p.w[idx] : 0.0f, e);
-      cnt += __syncthreads_count(e);
+      const size_t idx = first + (size_t)k * kRadThreads;
+      const bool in = idx < number;
+      cell[k] = in ? p.cell[idx] : AP_MAX_CELL;
+      flag[k] = in ? p.flag[idx] : 0u;
+      gam[k] = in ? p.E[idx] : 0.0f;
     }
-    if (threadIdx.x == 0) counts[ch] = (uint32_t)cnt;
+    bool want[kRadPer];
+#pragma unroll
+    for (int k = 0; k < kRadPer; ++k) {
+      int c1, c2;
+      want[k] = cell[k] != AP_MAX_CELL && bulk_cell(K.m, cell[k], c1, c2) &&
+                (flag[k] >> 29) != 2u && may_emit(K, gam[k]);
+    }
+    const uint32_t em = test_listed(L, (size_t)ch * kRadChunk, want, [&](size_t idx) {
+      if (K.model == AP_RAD_DEFAULT) return true;  // may_emit is its whole test
+      float u[4];
+      uniforms(K, 1u, ids[idx], u);
+      return check_emit(K, p, idx, p.cell[idx], u);
+    });
+#pragma unroll
+    for (int k = 0; k < kRadPer; ++k) {
+      const size_t idx = first + (size_t)k * kRadThreads;
+      const bool e = (em >> k) & 1u;
+      if (idx < number) mark[idx] = e ? 1 : 0;
+      if (K.produced.ptr) add_produced(K, cell[k], e ? p.w[idx] : 0.0f, e);
+    }
+    const uint32_t cnt = block_count(__popc(em));
+    if (threadIdx.x == 0) counts[ch] = cnt;
   }
 }
 
@@ -538,8 +646,12 @@ __global__ void __launch_bounds__(kRadThreads)
                       const uint32_t *offs, size_t number, size_t ph_base, size_t ph_cap,
                       uint64_t id0, uint32_t nchunks) {
   for (uint32_t ch = blockIdx.x; ch < nchunks; ch += gridDim.x) {
+    // nothing to write: no marks, or all of them past the capacity (their
+    // parents keep their energy)
+    const uint32_t r0 = offs[ch];
+    if (offs[ch + 1] == r0 || ph_base + r0 >= ph_cap) continue;
     uint32_t e4;
-    uint32_t rank = chunk_ranks(mark, number, ch, offs[ch], &e4);
+    uint32_t rank = chunk_ranks(mark, number, ch, r0, &e4);
     const size_t first = (size_t)ch * kRadChunk + (size_t)threadIdx.x * kRadPer;
 #pragma unroll 1
     for (int k = 0; k < kRadPer; ++k) {
@@ -561,31 +673,48 @@ __global__ void __launch_bounds__(kRadThreads)
 __global__ void __launch_bounds__(kRadThreads)
     k_rad_pair_mark(RadK K, PhK ph, size_t number, uint8_t *mark, uint32_t *counts,
                     uint32_t nchunks) {
+  __shared__ WarpList L;
   for (uint32_t ch = blockIdx.x; ch < nchunks; ch += gridDim.x) {
-    int cnt = 0;
-#pragma unroll 1
+    const size_t first = (size_t)ch * kRadChunk + threadIdx.x;
+    uint32_t cell[kRadPer];
+#pragma unroll
     for (int k = 0; k < kRadPer; ++k) {
-      const size_t idx = (size_t)ch * kRadChunk + (size_t)k * kRadThreads + threadIdx.x;
-      bool e = false;
-      uint32_t cell = AP_MAX_CELL;
-      if (idx < number) {
-        cell = ph.cell[idx];
-        if (cell != AP_MAX_CELL && in_bulk(K.m, cell)) {
-          if (K.model == AP_RAD_GR1D || K.model == AP_RAD_GAP1D) {
-            float u[4];
-            uniforms(K, 2u, ph.id[idx], u);
-            e = K.model == AP_RAD_GR1D ? check_pair_gr(K, ph, idx, cell, u)
-                                       : check_pair_gap(K, ph, idx, u);
-          } else {
-            e = check_pair(K, ph, idx, cell);
-          }
-        }
-        mark[idx] = e ? 1 : 0;
-      }
-      if (K.produced.ptr) add_produced(K, cell, e ? ph.w[idx] : 0.0f, e);
-      cnt += __syncthreads_count(e);
+      const size_t idx = first + (size_t)k * kRadThreads;
+      cell[k] = idx < number ? ph.cell[idx] : AP_MAX_CELL;
     }
-    if (threadIdx.x == 0) counts[ch] = (uint32_t)cnt;
+    bool want[kRadPer];
+#pragma unroll
+    for (int k = 0; k < kRadPer; ++k) {
+      int c1, c2;
+      want[k] = cell[k] != AP_MAX_CELL && bulk_cell(K.m, cell[k], c1, c2);
+    }
+    const uint32_t em = test_listed(L, (size_t)ch * kRadChunk, want, [&](size_t idx) {
+      if (K.model == AP_RAD_DEFAULT) return ph.path[idx] <= 0.0f;
+      const uint32_t c = ph.cell[idx];
+      if (K.model == AP_RAD_PULSAR) {
+        const float x1 = ph.x1[idx], x2 = ph.x2[idx];
+        const float p1 = ph.p1[idx], p2 = ph.p2[idx], p3 = ph.p3[idx], Eph = ph.E[idx];
+        int c1, c2;
+        bulk_cell(K.m, c, c1, c2);
+        bool gone;
+        const bool e = check_pair_pulsar(K, x1, x2, p1, p2, p3, Eph, c1, c2, gone);
+        if (gone) ph.cell[idx] = AP_MAX_CELL;
+        return e;
+      }
+      float u[4];
+      uniforms(K, 2u, ph.id[idx], u);
+      return K.model == AP_RAD_GR1D ? check_pair_gr(K, ph, idx, c, u)
+                                    : check_pair_gap(K, ph, idx, u);
+    });
+#pragma unroll
+    for (int k = 0; k < kRadPer; ++k) {
+      const size_t idx = first + (size_t)k * kRadThreads;
+      const bool e = (em >> k) & 1u;
+      if (idx < number) mark[idx] = e ? 1 : 0;
+      if (K.produced.ptr) add_produced(K, cell[k], e ? ph.w[idx] : 0.0f, e);
+    }
+    const uint32_t cnt = block_count(__popc(em));
+    if (threadIdx.x == 0) counts[ch] = cnt;
   }
 }
 
@@ -594,8 +723,10 @@ __global__ void __launch_bounds__(kRadThreads)
                       const uint32_t *offs, size_t number, size_t ptc_base, size_t ptc_cap,
                       uint64_t id0, uint32_t nchunks) {
   for (uint32_t ch = blockIdx.x; ch < nchunks; ch += gridDim.x) {
+    const uint32_t r0 = offs[ch];
+    if (offs[ch + 1] == r0) continue;  // no marks
     uint32_t e4;
-    uint32_t rank = chunk_ranks(mark, number, ch, offs[ch], &e4);
+    uint32_t rank = chunk_ranks(mark, number, ch, r0, &e4);
     const size_t first = (size_t)ch * kRadChunk + (size_t)threadIdx.x * kRadPer;
 #pragma unroll 1
     for (int k = 0; k < kRadPer; ++k) {
