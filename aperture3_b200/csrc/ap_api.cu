@@ -445,15 +445,8 @@ static int smooth_current_async(Ctx *c, uint32_t step) {
   int bnd[4] = {!c->params.periodic[0], !c->params.periodic[0], !c->params.periodic[1],
                 !c->params.periodic[1]};
   const bool out = ((step + 1) % (uint32_t)c->params.data_interval) == 0;
-  for (int it = 0; it < c->params.current_smoothing; ++it) {
-    for (int k = 0; k < 3; ++k) AP_TRY(launch_filter(*c, c->fields.J[k], bnd));
-    for (int k = 0; k < 3; ++k) AP_TRY(launch_copy_guards(*c, c->fields.J[k]));
-    if (out)
-      for (int s = 0; s < c->params.num_species; ++s) {
-        AP_TRY(launch_filter(*c, c->fields.Rho[s], bnd));
-        AP_TRY(launch_copy_guards(*c, c->fields.Rho[s]));
-      }
-  }
+  for (int it = 0; it < c->params.current_smoothing; ++it)
+    AP_TRY(launch_smooth_current(*c, out, bnd));
   return AP_OK;
 }
 
@@ -953,11 +946,7 @@ AP_API int ap_update_fields(ap_ctx *c, double dt, uint32_t step) {
     phase_end(c, ph);
     return finish(c);
   }
-  // field_solver::update_fields (field_solver.cu:334-358)
-  if (step == 0) AP_TRY(launch_update_e(*c, (float)(0.5 * dt)));
-  AP_TRY(launch_update_b(*c, (float)dt));
-  AP_TRY(launch_update_e(*c, (float)dt));
-  AP_TRY(launch_divs(*c));
+  AP_TRY(launch_fields(*c, (float)dt, step == 0 ? (float)(0.5 * dt) : 0.0f));
   phase_end(c, ph);
   return finish(c);
 }

@@ -348,7 +348,9 @@ cudaError_t launch_copy_guards(Ctx &c, ap_array a);
 cudaError_t launch_update_e(Ctx &c, float dt);
 cudaError_t launch_update_b(Ctx &c, float dt);
 cudaError_t launch_divs(Ctx &c);
+cudaError_t launch_fields(Ctx &c, float dt, float dt_half);
 cudaError_t launch_filter(Ctx &c, ap_array a, int bnd[4]);
+cudaError_t launch_smooth_current(Ctx &c, bool with_rho, const int bnd[4]);
 cudaError_t launch_zero(Ctx &c, ap_array a);
 cudaError_t launch_finalize_current(Ctx &c, int ncomp);
 cudaError_t launch_fixed_scale(Ctx &c);

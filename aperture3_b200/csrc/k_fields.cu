@@ -159,6 +159,52 @@ __global__ void k_divs(Geo G, Arr e1, Arr e2, Arr b1, Arr b2, Arr e01, Arr e02, 
   divs_cell(G, e1, e2, b1, b2, e01, e02, b01, b02, divE, divB, n1, n2);
 }
 
+// update_fields of a small grid (the optional half step of E, then B, E and
+// the divergences) in one launch: one cluster of eight CTAs, a cluster barrier
+// between the stages in place of a launch. Small CTAs, so that they find room
+// beside another run's push.
+constexpr int kSmallThreads = 256;
+constexpr int kSmallCtas = 8;
+constexpr int kSmallCells = 2 * kSmallThreads * kSmallCtas;
+
+__device__ __forceinline__ void cluster_barrier() {
+  asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+}
+
+struct FieldSet {
+  Arr e1, e2, e3, b1, b2, b3, e01, e02, e03, b01, b02, b03, j1, j2, j3, divE, divB;
+};
+
+__global__ void __cluster_dims__(kSmallCtas, 1, 1) __launch_bounds__(kSmallThreads)
+    k_fields_small(Geo G, const __grid_constant__ FieldSet F, float dt, float dt_half, int divs) {
+  const int first = blockIdx.x * kSmallThreads + threadIdx.x;
+  const int n = G.r0 * (G.dim > 1 ? G.r1 : 1);
+  const int y0 = G.dim > 1 ? G.g1 : 0;
+  auto each = [&](auto &&f) {
+    for (int t = first; t < n; t += kSmallThreads * kSmallCtas) {
+      const int y = t / G.r0;
+      f(G.g0 + t - y * G.r0, y0 + y);
+    }
+  };
+  auto e_step = [&](float h) {
+    each([&](int x, int y) {
+      e_update_cell(G, F.e1, F.e2, F.e3, F.b1, F.b2, F.b3, F.b01, F.b02, F.b03, F.j1, F.j2, F.j3,
+                    h, x, y);
+    });
+    cluster_barrier();
+  };
+  if (dt_half != 0.0f) e_step(dt_half);
+  each([&](int x, int y) {
+    b_update_cell(G, F.e1, F.e2, F.e3, F.e01, F.e02, F.e03, F.b1, F.b2, F.b3, dt, x, y);
+  });
+  cluster_barrier();
+  e_step(dt);
+  if (divs)
+    each([&](int x, int y) {
+      divs_cell(G, F.e1, F.e2, F.b1, F.b2, F.e01, F.e02, F.b01, F.b02, F.divE, F.divB, x, y);
+    });
+}
+
 // Guard strips of one dim: mode 0 copies interior strips into the opposite
 // guards (send_array_guard_cells_single_dir), mode 1 adds guard strips into
 // the opposite interior (send_add_array_guard_cells_single_dir). Both
@@ -189,10 +235,26 @@ __global__ void k_guard_strips(Arr a, int n0, int n1, int g, int dim, int mode) 
   }
 }
 
-// filter_current_cart_2d / _1d (ptc_updater.cu:501-560): bulk only.
-__global__ void k_filter(Geo G, Arr j, Arr t, int bl0, int bu0, int bl1, int bu1) {
+// One smoothing pass over several arrays (the current and, on output steps,
+// the charge densities) in two launches, blockIdx.z the array:
+// k_filter, filter_current_cart_2d / _1d (ptc_updater.cu:501-560), the bulk
+// only, into the scratch arrays; k_filter_store, the filtered bulk back and,
+// with `images`, every periodic guard cell as send_guard_cells leaves it
+// (dim 0 over all rows, then dim 1 over all columns): the value of its image,
+// which in a guard row of a non-periodic dim is that row's own, unfiltered,
+// value. Per array this was four launches (filter, copy, two guard strips), 20
+// for a current with two charge densities: 36 us of small kernels and their
+// launches on a 193^2 grid, which two launches replace.
+struct SmoothArrs {
+  Arr a[3 + AP_MAX_SPECIES];
+};
+
+__global__ void k_filter(Geo G, const __grid_constant__ SmoothArrs A, float *tmp, int tpitch,
+                         size_t tcomp, int bl0, int bu0, int bl1, int bu1) {
   const int a = G.g0 + blockIdx.x * blockDim.x + threadIdx.x;
   const int b = (G.dim > 1 ? G.g1 : 0) + blockIdx.y * blockDim.y + threadIdx.y;
+  const Arr j = A.a[blockIdx.z];
+  const Arr t{tmp + blockIdx.z * tcomp, tpitch};
   if (a >= G.n0 - G.g0) return;
   const int xp = (bu0 && a == G.n0 - G.g0 - 1) ? 0 : 1;
   const int xm = (bl0 && a == G.g0) ? 0 : 1;
@@ -218,12 +280,28 @@ __global__ void k_filter(Geo G, Arr j, Arr t, int bl0, int bu0, int bl1, int bu1
   }
 }
 
-__global__ void k_copy_bulk(Geo G, Arr src, Arr dst) {
-  const int a = G.g0 + blockIdx.x * blockDim.x + threadIdx.x;
-  const int b = (G.dim > 1 ? G.g1 : 0) + blockIdx.y * blockDim.y + threadIdx.y;
-  if (a >= G.n0 - G.g0) return;
-  if (G.dim > 1 && b >= G.n1 - G.g1) return;
-  dst(a, b) = src(a, b);
+__global__ void k_filter_store(Geo G, const float *__restrict__ tmp, int tpitch, size_t tcomp,
+                               const __grid_constant__ SmoothArrs A, int images) {
+  const int x = blockIdx.x * blockDim.x + threadIdx.x;
+  const int y = blockIdx.y * blockDim.y + threadIdx.y;
+  const int rows = G.dim > 1 ? G.n1 : 1;
+  if (x >= G.n0 || y >= rows) return;
+  const Arr a = A.a[blockIdx.z];
+  int xs = x, ys = y;  // the cell whose value this one takes
+  if (images && G.per0) {
+    if (x < G.g0) xs = x + G.r0;
+    else if (x >= G.n0 - G.g0) xs = x - G.r0;
+  }
+  if (images && G.dim > 1 && G.per1) {
+    if (y < G.g1) ys = y + G.r1;
+    else if (y >= G.n1 - G.g1) ys = y - G.r1;
+  }
+  const bool bulk = xs >= G.g0 && xs < G.n0 - G.g0 &&
+                    (G.dim == 1 || (ys >= G.g1 && ys < G.n1 - G.g1));
+  if (bulk)
+    a(x, y) = tmp[blockIdx.z * tcomp + (size_t)ys * tpitch + xs];
+  else if (xs != x || ys != y)
+    a(x, y) = a(xs, ys);
 }
 
 // Folds the periodic guard layers of the fixed-point accumulators into the
@@ -445,6 +523,28 @@ cudaError_t launch_update_b(Ctx &c, float dt) {
   return cudaGetLastError();
 }
 
+// field_solver::update_fields (field_solver.cu:334-358): B, E, divergences,
+// at step 0 after a half step of E. Grids of up to kSmallCells bulk cells take
+// one launch, larger ones a launch per stage.
+cudaError_t launch_fields(Ctx &c, float dt, float dt_half) {
+  const Geo G = make_geo(c);
+  const ap_fields &f = c.fields;
+  if ((size_t)G.r0 * (G.dim > 1 ? G.r1 : 1) <= (size_t)kSmallCells) {
+    const bool divs = f.divE.ptr && f.divB.ptr;
+    const FieldSet F{arr(f.E[0]),   arr(f.E[1]),   arr(f.E[2]),   arr(f.B[0]),   arr(f.B[1]),
+                     arr(f.B[2]),   arr(f.Ebg[0]), arr(f.Ebg[1]), arr(f.Ebg[2]), arr(f.Bbg[0]),
+                     arr(f.Bbg[1]), arr(f.Bbg[2]), arr(f.J[0]),   arr(f.J[1]),   arr(f.J[2]),
+                     divs ? arr(f.divE) : Arr{nullptr, 0}, divs ? arr(f.divB) : Arr{nullptr, 0}};
+    k_fields_small<<<kSmallCtas, kSmallThreads, 0, c.stream>>>(G, F, dt, dt_half, divs ? 1 : 0);
+    c.launches++;
+    return cudaGetLastError();
+  }
+  cudaError_t e = dt_half != 0.0f ? launch_update_e(c, dt_half) : cudaSuccess;
+  if (e == cudaSuccess) e = launch_update_b(c, dt);
+  if (e == cudaSuccess) e = launch_update_e(c, dt);
+  return e == cudaSuccess ? launch_divs(c) : e;
+}
+
 cudaError_t launch_divs(Ctx &c) {
   const ap_fields &f = c.fields;
   if (!f.divE.ptr || !f.divB.ptr) return cudaSuccess;
@@ -478,16 +578,37 @@ static cudaError_t guard_pass(Ctx &c, ap_array a, int mode) {
 cudaError_t launch_copy_guards(Ctx &c, ap_array a) { return guard_pass(c, a, 0); }
 cudaError_t launch_fold_guards(Ctx &c, ap_array a) { return guard_pass(c, a, 1); }
 
-cudaError_t launch_filter(Ctx &c, ap_array a, int bnd[4]) {
-  Geo G = make_geo(c);
+static cudaError_t smooth_pass(Ctx &c, const SmoothArrs &A, int narr, float *tmp, size_t tcomp,
+                               const int bnd[4], bool images) {
+  const Geo G = make_geo(c);
   dim3 grid, block;
   bulk_launch_shape(G, grid, block);
-  Arr t{c.tmp_j, c.tmp_pitch};
-  k_filter<<<grid, block, 0, c.stream>>>(G, arr(a), t, bnd[0], bnd[1], bnd[2], bnd[3]);
-  c.launches++;
-  k_copy_bulk<<<grid, block, 0, c.stream>>>(G, t, arr(a));
-  c.launches++;
+  grid.z = narr;
+  k_filter<<<grid, block, 0, c.stream>>>(G, A, tmp, G.n0, tcomp, bnd[0], bnd[1], bnd[2], bnd[3]);
+  const dim3 all((G.n0 + block.x - 1) / block.x,
+                 G.dim > 1 ? (G.n1 + block.y - 1) / block.y : 1, narr);
+  k_filter_store<<<all, block, 0, c.stream>>>(G, tmp, G.n0, tcomp, A, images ? 1 : 0);
+  c.launches += 2;
   return cudaGetLastError();
+}
+
+// The filter of one array alone, its guards as they are.
+cudaError_t launch_filter(Ctx &c, ap_array a, int bnd[4]) {
+  SmoothArrs A{};
+  A.a[0] = arr(a);
+  return smooth_pass(c, A, 1, c.tmp_j, 0, bnd, false);
+}
+
+// One smoothing pass of an update: J and, with_rho, the charge densities,
+// then their periodic guards. The scratch is the fixed-point accumulators'
+// memory: between the finalize and the next update they hold nothing.
+cudaError_t launch_smooth_current(Ctx &c, bool with_rho, const int bnd[4]) {
+  SmoothArrs A{};
+  int n = 0;
+  for (int k = 0; k < 3; ++k) A.a[n++] = arr(c.fields.J[k]);
+  if (with_rho)
+    for (int s = 0; s < c.params.num_species; ++s) A.a[n++] = arr(c.fields.Rho[s]);
+  return smooth_pass(c, A, n, reinterpret_cast<float *>(c.acc), 2 * c.acc_comp, bnd, true);
 }
 
 cudaError_t launch_finalize_current(Ctx &c, int ncomp) {
