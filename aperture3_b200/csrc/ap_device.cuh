@@ -34,6 +34,12 @@ __device__ __forceinline__ float cic(float dx) {
 //    otherwise c, c+1; the skipped node is at distance >= 1.
 // Skipping a node whose weight is exactly zero leaves the accumulated sum
 // bit-identical (the running sum starts at +0 and x + (+-0) == x).
+// With xc = fl(rel + c) and f = xc - c in [0, 1], a multiple of 2^-22 for a
+// bulk cell (2 <= c < 2^22), every difference and weight of interp_cell is
+// exact: the distances are f, 1 - f, |0.5 - f| and so on, so the weights are
+// 1 - f and f (stagger 1), and 0.5 -+ f or 1.5 - f, f - 0.5 (stagger 0), the
+// same bits as the reference's fl(1 - |node - xc|) in a third of the
+// instructions.
 struct Weights1D {
   int base0;       // first node for stagger 0 (c-1 or c)
   float w0[2];     // stagger-0 weights of nodes base0, base0 + 1
@@ -42,21 +48,42 @@ struct Weights1D {
 
 __device__ __forceinline__ Weights1D weights_1d(float rel, int c) {
   Weights1D W;
-  float xc = rel + (float)c;
-  float fc = (float)c;
-  float fcm = (float)(c - 1);
-  W.w1[0] = cic((fcm + 1.0f) - xc);
-  W.w1[1] = cic((fc + 1.0f) - xc);
-  if (xc < fc + 0.5f) {
-    W.base0 = c - 1;
-    W.w0[0] = cic((fcm + 0.5f) - xc);
-    W.w0[1] = cic((fc + 0.5f) - xc);
-  } else {
-    W.base0 = c;
-    W.w0[0] = cic((fc + 0.5f) - xc);
-    W.w0[1] = cic(((float)(c + 1) + 0.5f) - xc);
-  }
+  const float fc = (float)c;
+  const float f = (rel + fc) - fc;
+  W.w1[0] = 1.0f - f;
+  W.w1[1] = f;
+  const bool low = f < 0.5f;
+  W.base0 = low ? c - 1 : c;
+  W.w0[0] = (low ? 0.5f : 1.5f) - f;
+  W.w0[1] = f + (low ? 0.5f : -0.5f);
   return W;
+}
+
+// Quotients by one divisor b, each the correctly rounded a / b: y is the
+// correctly rounded reciprocal, a first quotient within two units is corrected
+// once to a faithful one, and a second correction with the exact remainder
+// rounds correctly (P. Markstein, "Computation of elementary functions on the
+// IBM RISC System/6000 processor", IBM J. Res. Dev. 34 (1990) 111-119). Signed
+// zeros come out as in the division. Valid for b in [1/2, 2^24) and a zero or
+// 2^-100 <= |a| <= 2^60: no intermediate leaves the normal range. Five fused
+// operations and no branch per quotient, against a reciprocal estimate,
+// its refinement and a slow-path branch for every plain division.
+struct SharedDiv {
+  float b, y;
+  __device__ __forceinline__ explicit SharedDiv(float d) : b(d), y(1.0f / d) {}
+  __device__ __forceinline__ float operator()(float a) const {
+    const float q0 = a * y;
+    const float q1 = __fmaf_rn(-__fmaf_rn(b, q0, -a), y, q0);
+    return __fmaf_rn(-__fmaf_rn(b, q1, -a), y, q1);
+  }
+};
+
+// Whether any of three numerators is nonzero and below 2^-100 in magnitude
+// (2 * bits - 1 drops the sign and sends zero to the top).
+__device__ __forceinline__ bool any_tiny(float a, float b, float c) {
+  const unsigned ua = 2u * __float_as_uint(a) - 1u, ub = 2u * __float_as_uint(b) - 1u,
+                 uc = 2u * __float_as_uint(c) - 1u;
+  return min(min(ua, ub), uc) < 0x1b000000u - 1u;
 }
 
 // vay_push (src/cuda/algorithms/vay_push.cuh:8-30). E and B are already
@@ -76,6 +103,53 @@ __device__ __forceinline__ void vay_push(float &p1, float &p2, float &p3, float 
   p1 = (up1 + B1 * ut * inv_gamma2 + (up2 * B3 - up3 * B2) / gamma) * s;
   p2 = (up2 + B2 * ut * inv_gamma2 + (up3 * B1 - up1 * B3) / gamma) * s;
   p3 = (up3 + B3 * ut * inv_gamma2 + (up1 * B2 - up2 * B1) / gamma) * s;
+}
+
+// vay_push followed by v = p / gamma, with the six quotients by the new gamma
+// through one reciprocal: the same bits. sigma + tt = 1 + up^2 and tt bound
+// every numerator from above; NaNs and numbers outside the bounds take the
+// plain divisions.
+__device__ __forceinline__ void vay_push_v(float &p1, float &p2, float &p3, float &gamma,
+                                           float E1, float E2, float E3, float B1, float B2,
+                                           float B3, float &v1, float &v2, float &v3) {
+  const float up1 = p1 + 2.0f * E1 + (p2 * B3 - p3 * B2) / gamma;
+  const float up2 = p2 + 2.0f * E2 + (p3 * B1 - p1 * B3) / gamma;
+  const float up3 = p3 + 2.0f * E3 + (p1 * B2 - p2 * B1) / gamma;
+  const float tt = B1 * B1 + B2 * B2 + B3 * B3;
+  const float ut = up1 * B1 + up2 * B2 + up3 * B3;
+  const float sigma = 1.0f + up1 * up1 + up2 * up2 + up3 * up3 - tt;
+  const float inv_gamma2 = 2.0f / (sigma + sqrtf(sigma * sigma + 4.0f * (tt + ut * ut)));
+  const float s = 1.0f / (1.0f + inv_gamma2 * tt);
+  gamma = 1.0f / sqrtf(inv_gamma2);
+  const float c1 = up2 * B3 - up3 * B2, c2 = up3 * B1 - up1 * B3, c3 = up1 * B2 - up2 * B1;
+  const float a1 = up1 + B1 * ut * inv_gamma2, a2 = up2 + B2 * ut * inv_gamma2,
+              a3 = up3 + B3 * ut * inv_gamma2;
+  const SharedDiv by_gamma(gamma);
+  // gamma < 2^24, |B| < 2^15, |up| < 2^31: numerators below 2^60
+  const bool bounded = gamma < 16777216.0f && gamma > 0.5f && tt < 1073741824.0f &&
+                       sigma < 4.6e18f;
+  float d1, d2, d3;
+  if (bounded && !any_tiny(c1, c2, c3)) {
+    d1 = by_gamma(c1);
+    d2 = by_gamma(c2);
+    d3 = by_gamma(c3);
+  } else {
+    d1 = c1 / gamma;
+    d2 = c2 / gamma;
+    d3 = c3 / gamma;
+  }
+  p1 = (a1 + d1) * s;
+  p2 = (a2 + d2) * s;
+  p3 = (a3 + d3) * s;
+  if (bounded && !any_tiny(p1, p2, p3)) {
+    v1 = by_gamma(p1);
+    v2 = by_gamma(p2);
+    v3 = by_gamma(p3);
+  } else {
+    v1 = p1 / gamma;
+    v2 = p2 / gamma;
+    v3 = p3 / gamma;
+  }
 }
 
 // movement2d / center2d (src/cuda/algorithms/ptc_updater_helper.cuh:26-41).

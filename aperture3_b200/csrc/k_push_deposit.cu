@@ -141,10 +141,21 @@ __device__ __forceinline__ void add_fixed(const Acc32 &a, int o, float v, float 
 // two commutes with rounding, so for a product a * b the value
 // (a * 2^S) * b equals (a * b) * 2^S bit for bit whenever the result is a
 // normal float; a result below the normal range rounds to X = 0 either way.
+// The low word takes all 32 low bits of X (mod 2^32): with H the sum of the
+// high words, the exact total is H * 2^L plus a remainder in [0, 2^32), which
+// the low sum gives mod 2^32 (fixed_total), so the low bits need no mask.
 __device__ __forceinline__ void add_fixed_scaled(const Acc32 &a, int o, float vs, int L) {
   const long long X = __float2ll_rn(vs);
   atomicAdd(a.hi + o, (int)(X >> L));
-  atomicAdd(a.lo + o, (unsigned)X & ((1u << L) - 1u));
+  atomicAdd(a.lo + o, (unsigned)X);
+}
+
+// The exact sum behind the two words of add_fixed_scaled: sum X = H * 2^L +
+// sum (X mod 2^L), the last sum below 2^32 for at most 2^lg contributions
+// (L = 32 - lg).
+__device__ __forceinline__ long long fixed_total(int H, unsigned lo, int L) {
+  const long long high = (long long)H * (1ll << L);
+  return high + (long long)(lo - (unsigned)high);
 }
 
 // Chunks of at most 256 particles are double-buffered: the loads of the
@@ -162,7 +173,7 @@ struct TileGeom {
   static constexpr int JX = TX + 4;   // J tile: two halo cells on each side
   static constexpr int JY = TY + 4;
   static constexpr int JSZ = JX * JY;
-  static constexpr int SP = CH + CH / 64;  // staged chunk, one pad word per 64
+  static constexpr int SP = CH + CH / 32;  // staged chunk, one pad word per 32
   static constexpr int HDR = 128;     // mbarrier, tile id, abort flag, counters
   static constexpr size_t stage_bytes() { return 10 * 4 * SP + 2 * SP; }
   static constexpr int NBUF = pipelined<CH>() ? 2 : 1;
@@ -174,7 +185,10 @@ struct TileGeom {
   }
 };
 
-__device__ __forceinline__ int spos(int e) { return e + (e >> 6); }
+// Lane l of a warp works on element l * CH / 32 + k: with one pad word per 32
+// elements the 32 lanes of a chunk of 256 (8 apart) fall into 32 banks, and so
+// do 32 consecutive elements of the coalesced loads and stores.
+__device__ __forceinline__ int spos(int e) { return e + (e >> 5); }
 
 // Write-back modes of a staged particle.
 constexpr uint8_t kWritePos = 1;  // x1, x2, x3, cell
@@ -416,6 +430,7 @@ __device__ __forceinline__ void push_deposit_tiles(const PushDepositParams &P0,
           const int sp = ptc_type(flag);
           float gamma = sqrtf(1.0f + p1 * p1 + p2 * p2 + p3 * p3);
           const bool em = !(flag & kFlagIgnoreEM);
+          float v1, v2, v3;
           // log-spherical: r at the particle (user_push_2d_logsph.cuh:36)
           float r_push = 0.0f;
           if constexpr (kLS) r_push = expf(mesh_pos(P.m.lower[0], P.m.delta[0], c1, g0, x1));
@@ -442,8 +457,10 @@ __device__ __forceinline__ void push_deposit_tiles(const PushDepositParams &P0,
               acc += row1[1] * wx1 * wy1;
               fe[q] = acc * qm;
             }
-            vay_push(p1, p2, p3, gamma, fe[0], fe[1], fe[2], fe[3], fe[4], fe[5]);
-            if constexpr (kLS) {
+            if constexpr (!kLS) {
+              vay_push_v(p1, p2, p3, gamma, fe[0], fe[1], fe[2], fe[3], fe[4], fe[5], v1, v2, v3);
+            } else {
+              vay_push(p1, p2, p3, gamma, fe[0], fe[1], fe[2], fe[3], fe[4], fe[5]);
               // gravity (gravity.cuh:12-26), applied with strength
               // dev_params.gravity on every push, then sync_kill_perp
               // when radiative cooling is on and the particle is no ion.
@@ -457,7 +474,11 @@ __device__ __forceinline__ void push_deposit_tiles(const PushDepositParams &P0,
           } else {
             gamma = P.p.E[s_idx[s]];  // the deposit reads the stored gamma
           }
-          float v1 = p1 / gamma, v2 = p2 / gamma, v3 = p3 / gamma;
+          if (kLS || !em) {
+            v1 = p1 / gamma;
+            v2 = p2 / gamma;
+            v3 = p3 / gamma;
+          }
           float nx1, nx2, nx3;
           int dc1, dc2;
           if constexpr (!kLS) {
@@ -519,59 +540,127 @@ __device__ __forceinline__ void push_deposit_tiles(const PushDepositParams &P0,
           const bool far = dc1 > 1 || dc1 < -1 || dc2 > 1 || dc2 < -1;
 
           if (!far && !(flag & kFlagIgnoreCurrent)) {
-            // Esirkepov over the reference's ranges i in [i0, i1], j in [j0, j1]
-            // (2 or 3 nodes per dim). Every lane walks the same 3 x 3 window
-            // starting at (ib, jb) so the warp does not diverge; the third
-            // node of a 2-node range is predicated off. Cumulative sums run
-            // in the reference's order, so each contribution keeps its value.
-            // The third column of J1 and the third row of J2 are only ever the
-            // last node of a 3-node range, where the cumulative sum covers the
-            // whole support (sum of new weights minus sum of old weights,
-            // zero up to rounding); the reference adds that rounding residue,
-            // these sites are skipped.
-            const float weight = -P.charge[sp] * w;
-            // the deposit's factors pre-scaled by 2^S (exact): weight, and
-            // -weight * v3 as the reference forms it before the site loop
-            const float wsc = weight * fscale;
-            const float w3s = -wsc * v3;
-            const int ib = (dc1 == -1 ? -2 : -1), nib = (dc1 == 0 ? 2 : 3);
-            const int jb = (dc2 == -1 ? -2 : -1), njb = (dc2 == 0 ? 2 : 3);
-            float sx0[3], sx1[3];
+            if constexpr (!kLS) {
+              // Esirkepov over the reference's ranges i in [i0, i1], j in [j0, j1]
+              // (2 or 3 nodes per dim). Every lane walks the same 3 x 3 window
+              // starting at (ib, jb) so the warp does not diverge; the third
+              // node of a 2-node range is predicated off. The decomposition is
+              // separable: with DX the cumulative sum of sx1 - sx0 along a row
+              // and YM the mean of sy0 and sy1, J1 of the face after node a in
+              // row b is -q w DX[a] YM[b]; J2 likewise; J3 is a sum of two
+              // products. The face after the last node of a range is not
+              // deposited: its cumulative sum covers the whole support (sum of
+              // new weights minus sum of old weights), zero up to rounding.
+              const float weight = -P.charge[sp] * w;
+              // the factors carry 2^S (exact), so that a product is the scaled
+              // contribution
+              const float wsc = weight * fscale;
+              const bool x3n = dc1 != 0, y3n = dc2 != 0;
+              const int ib = (dc1 == -1 ? -2 : -1), jb = (dc2 == -1 ? -2 : -1);
+              // old weights 1 - x, x on the nodes -1, 0; new ones 1 - nx, nx
+              // on -1 + dc, dc; the window starts at -2 for dc = -1, else -1
+              float sx0[3], sx1[3], sy0[3], sy1[3];
+              auto node_weights = [](float x, float nx, int dc, float s0[3], float s1[3]) {
+                const bool m = dc < 0, p = dc > 0;
+                const float r = 1.0f - x, nr = 1.0f - nx;
+                s0[0] = m ? 0.0f : r;
+                s0[1] = m ? r : x;
+                s0[2] = m ? x : 0.0f;
+                s1[0] = p ? 0.0f : nr;
+                s1[1] = p ? nr : nx;
+                s1[2] = p ? nx : 0.0f;
+              };
+              node_weights(x1, nx1, dc1, sx0, sx1);
+              node_weights(x2, nx2, dc2, sy0, sy1);
+              const Acc32 J1{sJhi, sJlo}, J2{sJhi + G::JSZ, sJlo + G::JSZ},
+                  J3{sJhi + 2 * G::JSZ, sJlo + 2 * G::JSZ};
+              const Acc32 R{sJhi + (3 + sp) * G::JSZ, sJlo + (3 + sp) * G::JSZ};
+              const bool rho = kRho && P.do_rho && sp < P.num_species;
+              const int o = (c2 + jb - jy0) * G::JX + (c1 + ib - jx0);
+              {
+                const float h = 0.5f * wsc;
+                // the cumulative sums from either end (the weights add up to 1)
+                const float d0 = sx1[0] - sx0[0], d1 = sx0[2] - sx1[2];
+                const float e0 = sy1[0] - sy0[0], e1 = sy0[2] - sy1[2];
+                const float dx[2] = {h * d0, h * d1}, dy[2] = {h * e0, h * e1};
 #pragma unroll
-            for (int a = 0; a < 3; ++a) {
-              const int i = ib + a;
-              sx0[a] = cic(-x1 + i + 1);
-              sx1[a] = cic(-nx1 + (i + 1 - dc1));
-            }
-            float djy[3] = {0.0f, 0.0f, 0.0f};
-            const Acc32 J1{sJhi, sJlo}, J2{sJhi + G::JSZ, sJlo + G::JSZ},
-                J3{sJhi + 2 * G::JSZ, sJlo + 2 * G::JSZ};
-            const Acc32 R{sJhi + (3 + sp) * G::JSZ, sJlo + (3 + sp) * G::JSZ};
-            const bool rho = kRho && P.do_rho && sp < P.num_species;
-            const int obase = (c2 + jb - jy0) * G::JX + (c1 + ib - jx0);
-#pragma unroll
-            for (int b = 0; b < 3; ++b) {
-              const int j = jb + b;
-              const bool jv = b < njb;
-              const float sy0 = cic(-x2 + j + 1);
-              const float sy1 = cic(-nx2 + (j + 1 - dc2));
-              float djx = 0.0f;
+                for (int b = 0; b < 3; ++b) {
+                  const float ym = sy0[b] + sy1[b], xm = sx0[b] + sx1[b];
+                  const bool yv = b < 2 || y3n, xv = b < 2 || x3n;
+                  if (yv) add_fixed_scaled(J1, o + b * G::JX + 1, dx[0] * ym, fx.L);
+                  if (yv && x3n) add_fixed_scaled(J1, o + b * G::JX + 2, dx[1] * ym, fx.L);
+                  if (xv) add_fixed_scaled(J2, o + G::JX + b, dy[0] * xm, fx.L);
+                  if (xv && y3n) add_fixed_scaled(J2, o + 2 * G::JX + b, dy[1] * xm, fx.L);
+                }
+              }
+              const float k3 = -wsc * v3 * 0.1666667f;
 #pragma unroll
               for (int a = 0; a < 3; ++a) {
-                if (jv && a < nib) {
-                  const int o = obase + b * G::JX + a;
-                  djx += movement2d(sy0, sy1, sx0[a], sx1[a]);
-                  if (a < 2) add_fixed_scaled(J1, o + 1, wsc * djx, fx.L);
-                  djy[a] += movement2d(sx0[a], sx1[a], sy0, sy1);
-                  if (b < 2) add_fixed_scaled(J2, o + G::JX, wsc * djy[a], fx.L);
-                  const float val2 = center2d(sx0[a], sx1[a], sy0, sy1);
-                  if constexpr (kLS)
+                const float c1w = k3 * (2.0f * sx1[a] + sx0[a]);
+                const float c0w = k3 * (sx1[a] + 2.0f * sx0[a]);
+                const float rw = -wsc * sx1[a];
+#pragma unroll
+                for (int b = 0; b < 3; ++b) {
+                  if ((a < 2 || x3n) && (b < 2 || y3n)) {
+                    const int s3 = o + b * G::JX + a;
+                    const float val = __fmaf_rn(c1w, sy1[b], c0w * sy0[b]);
+                    add_fixed_scaled(J3, s3, val, fx.L);
+                    if (rho) add_fixed_scaled(R, s3, rw * sy1[b], fx.L);
+                  }
+                }
+              }
+            } else {
+              // Esirkepov over the reference's ranges i in [i0, i1], j in [j0, j1]
+              // (2 or 3 nodes per dim). Every lane walks the same 3 x 3 window
+              // starting at (ib, jb) so the warp does not diverge; the third
+              // node of a 2-node range is predicated off. Cumulative sums run
+              // in the reference's order, so each contribution keeps its value.
+              // The third column of J1 and the third row of J2 are only ever the
+              // last node of a 3-node range, where the cumulative sum covers the
+              // whole support (sum of new weights minus sum of old weights,
+              // zero up to rounding); the reference adds that rounding residue,
+              // these sites are skipped.
+              const float weight = -P.charge[sp] * w;
+              // the deposit's factors pre-scaled by 2^S (exact): weight, and
+              // -weight * v3 as the reference forms it before the site loop
+              const float wsc = weight * fscale;
+              const float w3s = -wsc * v3;
+              const int ib = (dc1 == -1 ? -2 : -1), nib = (dc1 == 0 ? 2 : 3);
+              const int jb = (dc2 == -1 ? -2 : -1), njb = (dc2 == 0 ? 2 : 3);
+              float sx0[3], sx1[3];
+#pragma unroll
+              for (int a = 0; a < 3; ++a) {
+                const int i = ib + a;
+                sx0[a] = cic(-x1 + i + 1);
+                sx1[a] = cic(-nx1 + (i + 1 - dc1));
+              }
+              float djy[3] = {0.0f, 0.0f, 0.0f};
+              const Acc32 J1{sJhi, sJlo}, J2{sJhi + G::JSZ, sJlo + G::JSZ},
+                  J3{sJhi + 2 * G::JSZ, sJlo + 2 * G::JSZ};
+              const Acc32 R{sJhi + (3 + sp) * G::JSZ, sJlo + (3 + sp) * G::JSZ};
+              const bool rho = kRho && P.do_rho && sp < P.num_species;
+              const int obase = (c2 + jb - jy0) * G::JX + (c1 + ib - jx0);
+#pragma unroll
+              for (int b = 0; b < 3; ++b) {
+                const int j = jb + b;
+                const bool jv = b < njb;
+                const float sy0 = cic(-x2 + j + 1);
+                const float sy1 = cic(-nx2 + (j + 1 - dc2));
+                float djx = 0.0f;
+#pragma unroll
+                for (int a = 0; a < 3; ++a) {
+                  if (jv && a < nib) {
+                    const int o = obase + b * G::JX + a;
+                    djx += movement2d(sy0, sy1, sx0[a], sx1[a]);
+                    if (a < 2) add_fixed_scaled(J1, o + 1, wsc * djx, fx.L);
+                    djy[a] += movement2d(sx0[a], sx1[a], sy0, sy1);
+                    if (b < 2) add_fixed_scaled(J2, o + G::JX, wsc * djy[a], fx.L);
+                    const float val2 = center2d(sx0[a], sx1[a], sy0, sy1);
                     add_fixed_scaled(J3, o, w3s * val2 / s_dv[o], fx.L);
-                  else
-                    add_fixed_scaled(J3, o, w3s * val2, fx.L);
-                  if (rho) {
-                    const float s1 = sx1[a] * sy1;
-                    add_fixed_scaled(R, o, -wsc * s1, fx.L);
+                    if (rho) {
+                      const float s1 = sx1[a] * sy1;
+                      add_fixed_scaled(R, o, -wsc * s1, fx.L);
+                    }
                   }
                 }
               }
@@ -621,8 +710,12 @@ __device__ __forceinline__ void push_deposit_tiles(const PushDepositParams &P0,
         }
         s_dir[s] = (uint8_t)dir;
         s_mode[s] = mode;
-        const unsigned peers = __match_any_sync(__activemask(), dir);
-        if (lane == __ffs(peers) - 1) atomicAdd(&s_cnt[dir], (uint32_t)__popc(peers));
+        // direction counts: one add per warp for the particles that stay in
+        // the tile (nearly all), one per particle for the rest
+        const unsigned act = __activemask();
+        const unsigned stay = __ballot_sync(act, dir == 4u);
+        if (lane == __ffs(act) - 1) atomicAdd(&s_cnt[4], (uint32_t)__popc(stay));
+        if (dir != 4u) atomicAdd(&s_cnt[dir], 1u);
       }
       __syncthreads();
       // direction counts of this chunk, for the one-pass order update
@@ -679,7 +772,7 @@ __device__ __forceinline__ void push_deposit_tiles(const PushDepositParams &P0,
 
     // 4. flush the current (and charge) tile once
     for (int i = tid; i < nacc; i += kThreads2D) {
-      const long long v = (long long)sJhi[i] * (1ll << fx.L) + (long long)sJlo[i];
+      const long long v = fixed_total(sJhi[i], sJlo[i], fx.L);
       if (v == 0) continue;
       const int comp = i / G::JSZ, rem = i % G::JSZ;
       const int gx = jx0 + rem % G::JX, gy = jy0 + rem / G::JX;
@@ -912,6 +1005,7 @@ __device__ __forceinline__ void push_deposit_1d_chunk(const PushDepositParams &P
     const int c1 = (int)c;
     float gamma = sqrtf(1.0f + p1 * p1 + p2 * p2 + p3 * p3);
     const bool em = !(flag & kFlagIgnoreEM);
+    float v1, v2, v3;
     if (em) {
       // ptc_push_cart_1d (ptc_updater.cu:21-76): only the x stagger bit
       // matters in 1D.
@@ -920,18 +1014,20 @@ __device__ __forceinline__ void push_deposit_1d_chunk(const PushDepositParams &P
       float fe[6];
 #pragma unroll
       for (int q = 0; q < 6; ++q) fe[q] = interp_1d_global(P.F[q], W, c1, stag_x(q)) * qm;
-      vay_push(p1, p2, p3, gamma, fe[0], fe[1], fe[2], fe[3], fe[4], fe[5]);
+      vay_push_v(p1, p2, p3, gamma, fe[0], fe[1], fe[2], fe[3], fe[4], fe[5], v1, v2, v3);
       P.p.p1[idx] = p1;
       P.p.p2[idx] = p2;
       P.p.p3[idx] = p3;
       P.p.E[idx] = gamma;
     } else {
       gamma = P.p.E[idx];
+      v1 = p1 / gamma;
+      v2 = p2 / gamma;
+      v3 = p3 / gamma;
     }
     // deposit_current_cart_1d (ptc_updater.cu:220-293)
     const float w = cur.w;
     const float x2 = cur.x2, x3 = cur.x3;
-    const float v1 = p1 / gamma, v2 = p2 / gamma, v3 = p3 / gamma;
     float nx1 = x1 + (v1 * P.dt) / P.m.delta[0];
     const int dc1 = (int)floorf(nx1);
     nx1 -= (float)dc1;
