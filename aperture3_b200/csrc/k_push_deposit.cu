@@ -901,10 +901,10 @@ __device__ __forceinline__ void deposit_1d_node(bool act, int o, float a1, float
   }
 }
 
-// One chunk of kChunk1D particle slots of a 1D run: push, deposit into a
-// shared-memory window over the cells the chunk touches (or straight into
-// the global accumulators when the window would not fit), move.
-template <bool kRho>
+// One chunk of kThreads1D * kItems particle slots of a 1D run: push, deposit
+// into a shared-memory window over the cells the chunk touches (or straight
+// into the global accumulators when the window would not fit), move.
+template <bool kRho, int kItems = kItems1D>
 __device__ __forceinline__ void push_deposit_1d_chunk(const PushDepositParams &P, size_t ch,
                                                       int *sWhi, unsigned *sWlo, int &s_lo,
                                                       int &s_hi) {
@@ -920,16 +920,16 @@ __device__ __forceinline__ void push_deposit_1d_chunk(const PushDepositParams &P
   const FixedFmt fx = fixed_format(lgw, min(63 - 2 * lgw, 62 - lgn), P.qmax * *P.wmax);
   const float fscale = ldexpf(1.0f, fx.S);
   if (ch == 0 && tid == 0) *P.fx_used = fx;
-  const size_t first = ch * kChunk1D;
+  const size_t first = ch * (size_t)(kThreads1D * kItems);
   if (tid == 0) {
     s_lo = INT_MAX;
     s_hi = INT_MIN;
   }
   __syncthreads();
-  uint32_t cells[kItems1D];
+  uint32_t cells[kItems];
   int lo = INT_MAX, hi = INT_MIN;
 #pragma unroll
-  for (int k = 0; k < kItems1D; ++k) {
+  for (int k = 0; k < kItems; ++k) {
     const size_t idx = first + (size_t)k * kThreads1D + tid;
     cells[k] = idx < number ? P.p.cell[idx] : AP_MAX_CELL;
     if (cells[k] != AP_MAX_CELL) {
@@ -979,8 +979,8 @@ __device__ __forceinline__ void push_deposit_1d_chunk(const PushDepositParams &P
   Item1D cur{}, nxt{};
   load_item(0, cur);
 #pragma unroll 1
-  for (int k = 0; k < kItems1D; ++k) {
-    if (k + 1 < kItems1D) load_item(k + 1, nxt);
+  for (int k = 0; k < kItems; ++k) {
+    if (k + 1 < kItems) load_item(k + 1, nxt);
     // deposit inputs of this item; the deposit runs after the item, with
     // every lane of the warp present
     bool dep = false;
@@ -1108,15 +1108,16 @@ __device__ __forceinline__ void push_deposit_1d_chunk(const PushDepositParams &P
   __syncthreads();
 }
 
-template <bool kRho>
+template <bool kRho, int kItems>
 __global__ void __launch_bounds__(kThreads1D)
     k_push_deposit_1d(const __grid_constant__ PushDepositParams P) {
   __shared__ int sWhi[kWin1D];
   __shared__ unsigned sWlo[kWin1D];
   __shared__ int s_lo, s_hi;
-  const size_t nchunks = (P.number + kChunk1D - 1) / kChunk1D;
+  constexpr size_t kChunk = kThreads1D * kItems;
+  const size_t nchunks = (P.number + kChunk - 1) / kChunk;
   for (size_t ch = blockIdx.x; ch < nchunks; ch += gridDim.x)
-    push_deposit_1d_chunk<kRho>(P, ch, sWhi, sWlo, s_lo, s_hi);
+    push_deposit_1d_chunk<kRho, kItems>(P, ch, sWhi, sWlo, s_lo, s_hi);
 }
 
 // Many independent 1D runs in one launch: work item g is chunk
@@ -1323,16 +1324,33 @@ cudaError_t launch_selftest_wait(Ctx &c, uint32_t limit) {
   return cudaGetLastError();
 }
 
-cudaError_t launch_push_deposit_1d(Ctx &c, const PushDepositParams &P) {
-  size_t nchunks = (P.number + kChunk1D - 1) / kChunk1D;
+namespace {
+
+template <int kItems>
+cudaError_t launch_1d_items(Ctx &c, const PushDepositParams &P) {
+  const size_t chunk = (size_t)kThreads1D * kItems;
+  const size_t nchunks = (P.number + chunk - 1) / chunk;
   if (nchunks == 0) return cudaSuccess;
-  int grid = (int)(nchunks < (size_t)c.num_sms * 8 ? nchunks : (size_t)c.num_sms * 8);
+  const int grid = (int)(nchunks < (size_t)c.num_sms * 8 ? nchunks : (size_t)c.num_sms * 8);
   if (P.do_rho)
-    k_push_deposit_1d<true><<<grid, kThreads1D, 0, c.stream>>>(P);
+    k_push_deposit_1d<true, kItems><<<grid, kThreads1D, 0, c.stream>>>(P);
   else
-    k_push_deposit_1d<false><<<grid, kThreads1D, 0, c.stream>>>(P);
+    k_push_deposit_1d<false, kItems><<<grid, kThreads1D, 0, c.stream>>>(P);
   c.launches++;
   return cudaGetLastError();
+}
+
+}  // namespace
+
+// A chunk's slots per thread run one after the other, so few particles are cut
+// into shorter chunks until there are about four blocks per SM (the 48 KB
+// windows allow four).
+cudaError_t launch_push_deposit_1d(Ctx &c, const PushDepositParams &P) {
+  const size_t per = P.number / ((size_t)c.num_sms * 4 * kThreads1D);
+  if (per >= 4) return launch_1d_items<kItems1D>(c, P);
+  if (per >= 2) return launch_1d_items<4>(c, P);
+  if (per >= 1) return launch_1d_items<2>(c, P);
+  return launch_1d_items<1>(c, P);
 }
 
 }  // namespace apb
