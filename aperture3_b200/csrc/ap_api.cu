@@ -37,6 +37,21 @@ MeshK make_meshk(const ap_mesh &m) {
   return k;
 }
 
+cudaError_t alloc_control(Ctx &c) {
+  cudaFree(c.status);
+  c.status = nullptr;
+  c.queue = c.dir_count = nullptr;
+  const size_t bytes = kControlHead + sizeof(uint32_t) * ((size_t)c.tiles.ntiles * 10 + 16);
+  unsigned char *b = nullptr;
+  cudaError_t e = cudaMalloc(reinterpret_cast<void **>(&b), bytes);
+  if (e != cudaSuccess) return e;
+  static_assert(sizeof(DevStatus) + sizeof(uint32_t) <= kControlHead, "control head");
+  c.status = reinterpret_cast<DevStatus *>(b);
+  c.queue = reinterpret_cast<uint32_t *>(b + sizeof(DevStatus));
+  c.dir_count = reinterpret_cast<uint32_t *>(b + kControlHead);
+  return cudaMemset(b, 0, bytes);
+}
+
 }  // namespace apb
 
 namespace {
@@ -162,6 +177,19 @@ int check_status(Ctx *c) {
   return AP_OK;
 }
 
+// The 2D work-item list of the current tiles and particle capacity.
+int alloc_items(Ctx *c) {
+  if (c->mk.dim != 2) return AP_OK;
+  const size_t need = c->order_cap / (size_t)chunk_of(*c) + (size_t)c->tiles.ntiles + 2;
+  if (c->items_cap >= need) return AP_OK;
+  cudaFree(c->items);
+  c->items = nullptr;
+  c->items_cap = 0;
+  if (cudaMalloc(&c->items, need * sizeof(uint2)) != cudaSuccess) return AP_ERR_NOMEM;
+  c->items_cap = need;
+  return AP_OK;
+}
+
 int alloc_particle_state(Ctx *c, size_t cap) {
   if (cap <= c->order_cap && c->order[0]) return AP_OK;
   for (int i = 0; i < 2; ++i) {
@@ -175,6 +203,7 @@ int alloc_particle_state(Ctx *c, size_t cap) {
     if (cudaMalloc(&c->order[i], n * sizeof(uint32_t)) != cudaSuccess) return AP_ERR_NOMEM;
   if (cudaMalloc(&c->dir, n) != cudaSuccess) return AP_ERR_NOMEM;
   c->order_cap = n;
+  if (alloc_items(c) != AP_OK) return AP_ERR_NOMEM;
   // sort_by_cell's cell starts, here rather than at the first sort, so that
   // no allocation falls between the updates of a run
   if (!c->cell_start) {
@@ -264,28 +293,25 @@ AP_API int ap_ctx_create(const ap_mesh *mesh, const ap_params *params, ap_ctx **
   }
   c->own_stream = true;
   const int nt = c->tiles.ntiles;
-  bool ok = cudaMalloc(&c->status, sizeof(DevStatus)) == cudaSuccess &&
+  bool ok = alloc_control(*c) == cudaSuccess &&
             cudaMallocHost(&c->status_host, sizeof(DevStatus)) == cudaSuccess &&
-            cudaMalloc(&c->dir_count, sizeof(uint32_t) * ((size_t)nt * 10 + 16)) == cudaSuccess &&
             cudaMalloc(&c->grp_off, sizeof(uint32_t) * ((size_t)nt * 9 + 16)) == cudaSuccess &&
             cudaMalloc(&c->newcount, sizeof(uint32_t) * ((size_t)nt + 16)) == cudaSuccess &&
             cudaMalloc(&c->tile_start[0], sizeof(uint32_t) * (nt + 1)) == cudaSuccess &&
             cudaMalloc(&c->tile_start[1], sizeof(uint32_t) * (nt + 1)) == cudaSuccess &&
-            cudaMalloc(&c->queue, sizeof(uint32_t) * 4) == cudaSuccess &&
             cudaMalloc(&c->diag_dev, sizeof(double) * 16) == cudaSuccess &&
             cudaMalloc(&c->fx_used, sizeof(FixedFmt)) == cudaSuccess &&
-            cudaMalloc(&c->n_max, sizeof(uint32_t)) == cudaSuccess &&
+            cudaMalloc(&c->n_max, 3 * sizeof(uint32_t)) == cudaSuccess &&
             cudaMalloc(&c->wmax, sizeof(float)) == cudaSuccess &&
             cudaMallocHost(&c->diag_host, sizeof(double) * 16) == cudaSuccess;
   if (!ok) {
     ap_ctx_destroy(c);
     return AP_ERR_NOMEM;
   }
-  cudaMemset(c->status, 0, sizeof(DevStatus));
   cudaMemset(c->diag_dev, 0xFF, sizeof(double) * 16);  // NaN: nothing recorded yet
   std::memset(c->status_host, 0, sizeof(DevStatus));
   cudaMemset(c->fx_used, 0, sizeof(FixedFmt));
-  cudaMemset(c->n_max, 0, sizeof(uint32_t));
+  cudaMemset(c->n_max, 0, 3 * sizeof(uint32_t));
   cudaMemset(c->wmax, 0, sizeof(float));
   *out = c;
   return AP_OK;
@@ -301,16 +327,14 @@ AP_API int ap_ctx_destroy(ap_ctx *c) {
     cudaFree(c->vals[i]);
   }
   cudaFree(c->dir);
-  cudaFree(c->dir_count);
+  cudaFree(c->items);
   cudaFree(c->grp_off);
   cudaFree(c->newcount);
-  cudaFree(c->queue);
   cudaFree(c->rx_counts);
   cudaFree(c->gather_tmp);
   cudaFree(c->cell_start);
   cudaFree(c->cell_count);
   cudaFree(c->chunk_count);
-  cudaFree(c->big_tiles);
   cudaFree(c->ls_surface);
   cudaFree(c->sort_max);
   cudaFree(c->tmp_j);
@@ -650,7 +674,13 @@ int update_prepare(Ctx *c, double dt, uint32_t step, PushDepositParams &P, bool 
     for (int s = 0; s < pr.num_species; ++s) AP_TRY(launch_zero(*c, c->fields.Rho[s]));
     c->rho_is_zero = true;
   }
-  if (!batched) AP_TRY(cudaMemsetAsync(c->status, 0, sizeof(DevStatus), c->stream));
+  // status, queue and, in 2D, the direction counts the push adds to
+  if (!batched)
+    AP_TRY(cudaMemsetAsync(c->status, 0,
+                           c->mk.dim == 2 ? kControlHead + sizeof(uint32_t) * 10 *
+                                                               (size_t)c->tiles.ntiles
+                                          : kControlHead,
+                           c->stream));
   // continuity check: rho(t) of the previous update, before it is replaced
   c->cont_snap = false;
   if (c->cont_on && !batched && !ls && do_rho && c->last_rho_step == (long long)step - 1) {
@@ -744,13 +774,6 @@ int update_prepare(Ctx *c, double dt, uint32_t step, PushDepositParams &P, bool 
           AP_TRY(cudaMalloc(&c->chunk_count, sizeof(uint32_t) * 10 * need));
           c->chunk_count_cap = need;
         }
-        if (c->big_tiles_cap < (size_t)c->tiles.ntiles + 1) {
-          cudaFree(c->big_tiles);
-          c->big_tiles = nullptr;
-          c->big_tiles_cap = 0;
-          AP_TRY(cudaMalloc(&c->big_tiles, sizeof(uint32_t) * (c->tiles.ntiles + 1)));
-          c->big_tiles_cap = c->tiles.ntiles + 1;
-        }
         P.chunk_count = c->chunk_count;
         c->chunk_count_ok = true;
       }
@@ -759,6 +782,8 @@ int update_prepare(Ctx *c, double dt, uint32_t step, PushDepositParams &P, bool 
       P.tile_start = c->tile_start[c->cur];
       P.dir = c->dir;
       P.dir_count = c->dir_count;
+      P.items = c->items;
+      P.n_items = c->n_max + 1;
       P.queue = c->queue;
     }
   }
@@ -1399,13 +1424,13 @@ AP_API int ap_set_tile_shape(ap_ctx *c, int tx, int ty) {
   c->params.tile[1] = ty;
   choose_tiles(*c);
   const size_t nt = (size_t)c->tiles.ntiles;
-  cudaFree(c->dir_count);
   cudaFree(c->grp_off);
   cudaFree(c->newcount);
   cudaFree(c->tile_start[0]);
   cudaFree(c->tile_start[1]);
-  c->dir_count = c->grp_off = c->newcount = c->tile_start[0] = c->tile_start[1] = nullptr;
-  AP_TRY(cudaMalloc(&c->dir_count, sizeof(uint32_t) * (nt * 10 + 16)));
+  c->grp_off = c->newcount = c->tile_start[0] = c->tile_start[1] = nullptr;
+  AP_TRY(alloc_control(*c));
+  if (c->order_cap) AP_TRY_ST(alloc_items(c));
   AP_TRY(cudaMalloc(&c->grp_off, sizeof(uint32_t) * (nt * 9 + 16)));
   AP_TRY(cudaMalloc(&c->newcount, sizeof(uint32_t) * (nt + 16)));
   AP_TRY(cudaMalloc(&c->tile_start[0], sizeof(uint32_t) * (nt + 1)));

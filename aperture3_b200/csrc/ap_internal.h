@@ -95,6 +95,10 @@ struct PushDepositParams {
   const uint32_t *tile_start;
   uint8_t *dir;
   uint32_t *dir_count;   // ntiles * 10
+  // work items: item k is list entries [items[k].y, items[k].y + item_len) of
+  // tile items[k].x
+  const uint2 *items;
+  const uint32_t *n_items;  // [0] their number, [1] item_len, a multiple of the chunk
   // per staged chunk of the tile lists, its direction counts (10 each):
   // chunk k of tile t is entry tile_start[t] / CH + t + k (null: not kept)
   uint32_t *chunk_count;
@@ -208,16 +212,22 @@ struct Ctx {
   int cur = 0;
   bool order_valid = false;
   uint8_t *dir = nullptr;
+  // one block, cleared by one memset per update: the status, the work queue
+  // and the per-tile direction counts
   uint32_t *dir_count = nullptr;
   uint32_t *grp_off = nullptr;
   uint32_t *newcount = nullptr;  // per-tile population after the step
   uint32_t *queue = nullptr;
   size_t order_cap = 0;
+  // work items of the 2D push / deposit (PushDepositParams::items), rebuilt
+  // with every tile order
+  uint2 *items = nullptr;
+  size_t items_cap = 0;
+  uint32_t item_len = 1;         // entries per item of the last list
+  size_t item_total = 0;         // in a batch: particles of all its 2D runs
   // per-chunk direction counts of the push / deposit (one-pass order update)
   uint32_t *chunk_count = nullptr;
   size_t chunk_count_cap = 0;  // entries of 10 counts
-  uint32_t *big_tiles = nullptr;  // count, then tiles left to the two-pass kernel
-  size_t big_tiles_cap = 0;
   bool chunk_count_ok = false;  // the last push / deposit recorded them
 
   // rebuild / sort scratch
@@ -234,7 +244,7 @@ struct Ctx {
   unsigned long long *acc = nullptr;
   size_t acc_comp = 0;
   FixedFmt *fx_used = nullptr;  // device: format of the last deposit
-  uint32_t *n_max = nullptr;    // device: largest tile population
+  uint32_t *n_max = nullptr;    // device: largest tile population, number of work items, item length
   float *wmax = nullptr;        // device: max |weight| over the bound particles
   bool scale_valid = false;
 
@@ -306,7 +316,7 @@ struct Ctx {
   int ev_used = 0, ev_cap = 0;
   uint64_t pd_launches = 0;
 
-  DevStatus *status = nullptr;     // device
+  DevStatus *status = nullptr;     // device (start of the control block)
   DevStatus *status_host = nullptr;  // pinned
   double *diag_dev = nullptr;
   double *diag_host = nullptr;
@@ -322,13 +332,14 @@ struct Ctx {
 cudaError_t launch_push_deposit_2d(Ctx &c, const PushDepositParams &P);
 cudaError_t launch_push_deposit_1d(Ctx &c, const PushDepositParams &P);
 cudaError_t launch_selftest_wait(Ctx &c, uint32_t limit);
-cudaError_t launch_tile_scan(Ctx &c, const uint32_t *dir_count,
-                             uint32_t *new_start, uint32_t *grp_off);
+// Populations and offsets of the tiles after a push, from its direction
+// counts, and the offset of every (source tile, direction) group.
+cudaError_t launch_tile_scan(Ctx &c, const uint32_t *dir_count, uint32_t *new_start,
+                             uint32_t *grp_off);
 // old_order null: the particle at list position p sits in slot slot0 + p.
-cudaError_t launch_order_scatter(Ctx &c, const uint32_t *old_start,
-                                 const uint32_t *old_order, const uint8_t *dir,
-                                 const uint32_t *grp_off, uint32_t *new_order,
-                                 uint32_t slot0 = 0);
+cudaError_t launch_order_scatter(Ctx &c, const uint32_t *old_start, const uint32_t *old_order,
+                                 const uint8_t *dir, const uint32_t *grp_off,
+                                 uint32_t *new_order, uint32_t slot0 = 0);
 cudaError_t rebuild_tile_order(Ctx &c);
 // Stable LSD radix sort of (c.keys[0], c.vals[0])[0, n) by the low end_bit
 // bits of the keys, ping-ponging with keys[1] / vals[1] (k_radix.cu).
@@ -441,6 +452,11 @@ int update_smooth(Ctx *c, uint32_t step);
 int fill_run1d(Ctx *c, double dt, uint32_t step, Run1D &d);
 
 int ctx_check_status(Ctx *c);
+
+// The control block of a context: status, queue, direction counts of ntiles
+// tiles. Allocates (or replaces) it and clears it.
+cudaError_t alloc_control(Ctx &c);
+constexpr size_t kControlHead = 64;  // bytes before the direction counts
 
 // One persistent push / deposit launch over the tiles of several 2D
 // Cartesian runs with the same tile shape, chunk and field-load path.

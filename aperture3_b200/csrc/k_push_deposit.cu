@@ -97,10 +97,6 @@ __device__ __forceinline__ void cp_async4(void *smem_dst, const void *gmem_src) 
                : "memory");
 }
 
-__device__ __forceinline__ void cp_async_wait_all() {
-  asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
-}
-
 __device__ __forceinline__ void cp_async_commit() {
   asm volatile("cp.async.commit_group;" ::: "memory");
 }
@@ -246,6 +242,7 @@ __device__ __forceinline__ void push_deposit_tiles(const PushDepositParams &P0,
     const int g = *s_tile;
     const CUtensorMap *mp = maps0;
     int t = g;
+    uint32_t item0 = 0;  // this work item's first list entry of the tile
     if constexpr (kMulti) {
       if ((uint32_t)g >= base[nruns]) break;
       int lo = 0, hi = nruns - 1;  // largest r with base[r] <= g
@@ -261,7 +258,10 @@ __device__ __forceinline__ void push_deposit_tiles(const PushDepositParams &P0,
       mp = runs[lo].maps.m;
       t = g - (int)base[lo];
     } else {
-      if (g >= P0.t.ntiles) break;
+      if ((uint32_t)g >= *P0.n_items) break;
+      const uint2 it = P0.items[g];
+      t = (int)it.x;
+      item0 = it.y;
     }
     const PushDepositParams &P =
         kMulti ? *reinterpret_cast<const PushDepositParams *>(s_pbuf) : P0;
@@ -284,7 +284,7 @@ __device__ __forceinline__ void push_deposit_tiles(const PushDepositParams &P0,
     const int lg = max(4, bits_of(*P.n_max));
     const FixedFmt fx = fixed_format(lg, 63 - 2 * lg, P.qmax * *P.wmax);
     const float fscale = ldexpf(1.0f, fx.S);
-    if (t == 0 && tid == 0) *P.fx_used = fx;
+    if ((kMulti ? t : g) == 0 && tid == 0) *P.fx_used = fx;
 
     const int tix = t % P.t.ntx, tiy = t / P.t.ntx;
     const int x0 = g0 + tix * TX, y0 = g1 + tiy * TY;
@@ -295,7 +295,9 @@ __device__ __forceinline__ void push_deposit_tiles(const PushDepositParams &P0,
     // indices run two chunks ahead (slot (chunk index) & 1 of s_ord), so
     // the gathers of the next chunk never wait for them
     const uint32_t base = P.tile_start[t];
-    const int n_t = (int)(P.tile_start[t + 1] - base);
+    const int n_tile = (int)(P.tile_start[t + 1] - base);
+    const int p0 = (int)item0;
+    const int n_t = kMulti ? n_tile : min(n_tile, p0 + (int)P.n_items[1]);  // end of the item
     auto prefetch_order = [&](int c0) {
       uint32_t *dst = s_ord + ((c0 / CH) & 1) * CH;
       const int nch = min(CH, n_t - c0);
@@ -303,8 +305,8 @@ __device__ __forceinline__ void push_deposit_tiles(const PushDepositParams &P0,
       cp_async_commit();
     };
     if (G::NBUF == 2) {
-      if (n_t > 0) prefetch_order(0);
-      if (CH < n_t) prefetch_order(CH);
+      if (p0 < n_t) prefetch_order(p0);
+      if (p0 + CH < n_t) prefetch_order(p0 + CH);
     }
 
     // 1. field tile
@@ -377,12 +379,12 @@ __device__ __forceinline__ void push_deposit_tiles(const PushDepositParams &P0,
     };
     int buf = 0;
     uint32_t cnt_prev = 0;  // threads < 10: the tile's direction count so far
-    if (G::NBUF == 2 && n_t > 0) {
-      issue(0, 0);
+    if (G::NBUF == 2 && p0 < n_t) {
+      issue(p0, 0);
       cp_async_wait_group<0>();
       __syncthreads();
     }
-    for (int c0 = 0; c0 < n_t; c0 += CH) {
+    for (int c0 = p0; c0 < n_t; c0 += CH) {
       const int nch = min(CH, n_t - c0);
       if (G::NBUF == 2) {
         // this chunk landed at the end of the previous one; start the next
@@ -780,7 +782,12 @@ __device__ __forceinline__ void push_deposit_tiles(const PushDepositParams &P0,
       atomicAdd(P.acc + comp * P.acc_comp + (size_t)gy * P.acc_pitch + gx,
                 (unsigned long long)v);
     }
-    if (tid < 10) P.dir_count[t * 10 + tid] = s_cnt[tid];
+    if (tid < 10) {
+      if constexpr (kMulti)
+        P.dir_count[t * 10 + tid] = s_cnt[tid];
+      else if (s_cnt[tid])
+        atomicAdd(&P.dir_count[t * 10 + tid], s_cnt[tid]);  // a tile's items, counts start at 0
+    }
     phase ^= 1u;
   }
 }
@@ -1153,9 +1160,7 @@ template <int TX, int TY, int CH, int MINB, bool kLS = false>
 cudaError_t launch_2d_tiles(Ctx &c, const PushDepositParams &P) {
   using G = TileGeom<TX, TY, CH>;
   const int nrho = P.do_rho ? P.num_species : 0;
-  const size_t smem = G::smem_bytes(nrho, kLS);
-  cudaError_t e = cudaMemsetAsync(P.queue, 0, sizeof(uint32_t), c.stream);
-  if (e != cudaSuccess) return e;
+  const size_t smem = G::smem_bytes(nrho, kLS);  // the queue was cleared with the status
   auto run = [&](auto kern) -> cudaError_t {
     cudaError_t err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                            (int)smem);
@@ -1164,10 +1169,11 @@ cudaError_t launch_2d_tiles(Ctx &c, const PushDepositParams &P) {
     err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kThreads2D, smem);
     if (err != cudaSuccess) return err;
     if (per_sm < 1) return cudaErrorInvalidConfiguration;
-    int grid = c.num_sms * per_sm;
-    if (grid > P.t.ntiles) grid = P.t.ntiles;
+    size_t grid = (size_t)c.num_sms * per_sm;
+    const size_t items = P.t.ntiles + (c.number - c.store_base) / c.item_len;  // at most
+    if (grid > items) grid = items;
     if (grid < 1) grid = 1;
-    kern<<<grid, kThreads2D, smem, c.stream>>>(P, c.maps);
+    kern<<<(int)grid, kThreads2D, smem, c.stream>>>(P, c.maps);
     c.launches++;
     return cudaGetLastError();
   };

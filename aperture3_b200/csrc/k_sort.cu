@@ -6,11 +6,12 @@
 // direction counts. Because the input is grouped by tile and a particle
 // only moves to one of its tile's eight neighbours, the stable counting
 // sort by new tile reduces to:
-//   k_tile_newcount / k_scan_counts / k_tile_groups: for each destination
-//                   tile, sum the counts from its (up
-//                   to nine) source tiles, scan to get tile offsets, and
-//                   give each (source, direction) group its offset, sources
-//                   taken in ascending tile index;
+//   k_tile_newcount / k_scan_counts (one launch up to 1024 tiles): for each
+//                   destination tile, sum the counts from its (up to nine)
+//                   source tiles and scan the sums to get tile offsets;
+//   k_tile_groups   gives each (source, direction) group its offset in the
+//                   destination tile, sources in ascending tile index (part
+//                   of the scan's launch up to 113 tiles);
 //   k_order_scatter for each source tile, rank particles within their
 //                   direction group in order and write them to
 //                   group offset + rank.
@@ -56,299 +57,267 @@ __device__ __forceinline__ int source_tile(const TileTopo &T, int ux, int uy, in
   return sx + sy * T.ntx;
 }
 
-// Gathers the (source tile, direction, count) triples of destination u,
-// sorted by source tile index. Returns how many there are.
-__device__ __forceinline__ int gather_sources(const TileTopo &T, const uint32_t *cnt, int u,
-                                              int src[9], int dirv[9], uint32_t num[9]) {
+// New population of destination tile u: the counts its (up to nine) source
+// tiles recorded for the direction that leads to it.
+__device__ __forceinline__ uint32_t new_population(const TileTopo &T, const uint32_t *cnt, int u) {
   const int ux = u % T.ntx, uy = u / T.ntx;
-  int n = 0;
-  for (int dy = -1; dy <= 1; ++dy)
-    for (int dx = -1; dx <= 1; ++dx) {
-      const int s = source_tile(T, ux, uy, dx, dy);
-      if (s < 0) continue;
-      const int d = (dy + 1) * 3 + (dx + 1);
-      // insertion by source index
-      int k = n++;
-      while (k > 0 && src[k - 1] > s) {
-        src[k] = src[k - 1];
-        dirv[k] = dirv[k - 1];
-        num[k] = num[k - 1];
-        --k;
-      }
-      src[k] = s;
-      dirv[k] = d;
-      num[k] = cnt[s * 10 + d];
-    }
-  return n;
-}
-
-// New population of every destination tile: the counts its (up to nine)
-// source tiles recorded for the direction that leads to it.
-__global__ void k_tile_newcount(TileTopo T, const uint32_t *__restrict__ cnt,
-                                uint32_t *__restrict__ newcount) {
-  for (int u = blockIdx.x * blockDim.x + threadIdx.x; u < T.ntiles; u += gridDim.x * blockDim.x) {
-    int src[9], dirv[9];
-    uint32_t num[9];
-    const int n = gather_sources(T, cnt, u, src, dirv, num);
-    uint32_t nu = 0;
-    for (int k = 0; k < n; ++k) nu += num[k];
-    newcount[u] = nu;
+  uint32_t nu = 0;
+#pragma unroll
+  for (int d = 0; d < 9; ++d) {
+    const int s = source_tile(T, ux, uy, d % 3 - 1, d / 3 - 1);
+    if (s >= 0) nu += cnt[s * 10 + d];
   }
+  return nu;
 }
 
-// Offsets of the (source, direction) groups inside each destination tile:
-// sources in ascending tile index, so the concatenation is the stable order.
+// Position of the first entry of group (source tile s, direction d) in the
+// new order: inside the destination tile the groups stand by ascending
+// source tile, those of one source by ascending direction.
+__device__ __forceinline__ uint32_t group_offset(const TileTopo &T, const uint32_t *cnt,
+                                                 const uint32_t *new_start, int s, int d) {
+  const int sx = s % T.ntx, sy = s / T.ntx;
+  int ux = sx + d % 3 - 1, uy = sy + d / 3 - 1;
+  if (ux < 0 || ux >= T.ntx) {
+    if (!T.per0) return 0;  // an empty group
+    ux += ux < 0 ? T.ntx : -T.ntx;
+  }
+  if (uy < 0 || uy >= T.nty) {
+    if (!T.per1) return 0;
+    uy += uy < 0 ? T.nty : -T.nty;
+  }
+  uint32_t off = new_start[ux + uy * T.ntx];
+#pragma unroll
+  for (int e = 0; e < 9; ++e) {
+    const int o = source_tile(T, ux, uy, e % 3 - 1, e / 3 - 1);
+    if (o >= 0 && (o < s || (o == s && e < d))) off += cnt[o * 10 + e];
+  }
+  return off;
+}
+
+// One thread per (tile, direction): 2 us on 4096 tiles, where one thread per
+// tile, sorting its nine sources in local memory, took 7 us (6 us on 16
+// tiles). Computing the offsets inside the scatter's blocks was slower: the
+// chain of loads stands before every tile's walk (65 -> 100 us on 16384
+// tiles of 1000 particles).
 __global__ void k_tile_groups(TileTopo T, const uint32_t *__restrict__ cnt,
                               const uint32_t *__restrict__ new_start,
                               uint32_t *__restrict__ grp_off) {
-  for (int u = blockIdx.x * blockDim.x + threadIdx.x; u < T.ntiles; u += gridDim.x * blockDim.x) {
-    int src[9], dirv[9];
-    uint32_t num[9];
-    const int n = gather_sources(T, cnt, u, src, dirv, num);
-    uint32_t run = new_start[u];
-    for (int k = 0; k < n; ++k) {
-      grp_off[src[k] * 9 + dirv[k]] = run;
-      run += num[k];
-    }
-  }
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < T.ntiles * 9) grp_off[i] = group_offset(T, cnt, new_start, i / 9, i % 9);
 }
 
-// One CTA per source tile: stable rank within each direction group. The
-// tile's list is cut into one contiguous segment per warp; pass 1 counts the
-// directions of each segment (each lane adds its entries into packed
-// per-direction counters, summed over the warp at the end), one barrier
-// turns the counts into per-warp offsets, and pass 2 walks the segment
-// again 32 entries at a time, ranking lanes that share a direction (a
-// ballot for the entries that stay in the tile, nearly all of them;
-// __match_any_sync for the rest), so every entry lands at group offset +
-// entries of that direction before it. Both passes issue the loads of four
+__global__ void k_tile_newcount(TileTopo T, const uint32_t *__restrict__ cnt,
+                                uint32_t *__restrict__ newcount) {
+  for (int u = blockIdx.x * blockDim.x + threadIdx.x; u < T.ntiles; u += gridDim.x * blockDim.x)
+    newcount[u] = new_population(T, cnt, u);
+}
+
+// Stable placement of one source tile's entries [b, e) in the new order by
+// two passes over them: the list is cut into one contiguous segment per
+// warp; pass 1 counts the directions of each segment (each lane adds its
+// entries into packed per-direction counters, summed over the warp at the
+// end), one barrier turns the counts into per-warp offsets, and pass 2 walks
+// the segment again 32 entries at a time, ranking lanes that share a
+// direction (a ballot for the entries that stay in the tile, nearly all of
+// them; __match_any_sync for the rest), so every entry lands at group offset
+// + entries of that direction before it. Both passes issue the loads of four
 // 32-entry steps before using them.
-__global__ void __launch_bounds__(kScatterThreads)
-    k_order_scatter(int ntiles, const uint32_t *__restrict__ old_start,
-                    const uint32_t *__restrict__ old_order, const uint8_t *__restrict__ dir,
-                    const uint32_t *__restrict__ grp_off, uint32_t *__restrict__ new_order,
-                    uint32_t capacity, uint32_t slot0, const uint32_t *__restrict__ tile_list,
-                    DevStatus *status) {
-  constexpr int kWarps = kScatterThreads / 32;
-  constexpr int kU = 4;  // 32-entry steps per batch of loads
-  __shared__ uint32_t s_cnt[kWarps][10];
-  __shared__ uint32_t s_base[kWarps][10];
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+struct ScatterOut {
+  const uint32_t *old_order;  // null: the particle at list position p sits in slot slot0 + p
+  const uint8_t *dir;
+  uint32_t *new_order;
+  uint32_t capacity, slot0;
+  DevStatus *status;
+};
+
+constexpr int kScatterWarps = kScatterThreads / 32;
+constexpr int kScatterU = 4;  // 32-entry steps per batch of loads
+
+// Places entries [w0, w1) of one warp in order; s_base[d] holds the position
+// of the next entry of each direction.
+__device__ __forceinline__ void scatter_walk(const ScatterOut &S, uint32_t w0, uint32_t w1,
+                                             uint32_t *s_base) {
+  const int lane = threadIdx.x & 31;
   const uint32_t lt = (1u << lane) - 1u;
-  // all tiles, or the count and indices in tile_list
-  const int nlist = tile_list ? (int)tile_list[0] : ntiles;
-  for (int li = blockIdx.x; li < nlist; li += gridDim.x) {
-    const int s = tile_list ? (int)tile_list[1 + li] : li;
-    const uint32_t b = old_start[s], e = old_start[s + 1];
-    const uint32_t n = e - b;
-    const uint32_t seg = ((n + kWarps * 32 - 1) / (kWarps * 32)) * 32;
-    const uint32_t w0 = b + min(n, warp * seg), w1 = b + min(n, (warp + 1) * seg);
-    // pass 1: direction counts of this warp's segment; packed counters of
-    // 16 bits, directions 0-3 in c0, 4-7 in c1, 8-9 in c2, summed over the
-    // warp into lane f's mycnt every 256 batches (at most 32 x 4 x 256 =
-    // 32768 entries per counter in between)
-    unsigned long long c0 = 0, c1 = 0, c2 = 0;
-    uint32_t mycnt = 0;  // lane f < 10: count of direction f
-    auto flush = [&]() {
+  uint32_t base4 = s_base[4];
+  for (uint32_t q = w0; q < w1; q += 32 * kScatterU) {
+    uint32_t d[kScatterU], src[kScatterU];
 #pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
-        c0 += __shfl_xor_sync(0xffffffffu, c0, o);
-        c1 += __shfl_xor_sync(0xffffffffu, c1, o);
-        c2 += __shfl_xor_sync(0xffffffffu, c2, o);
-      }
-      const unsigned long long w = lane < 4 ? c0 : (lane < 8 ? c1 : c2);
-      if (lane < 10) mycnt += (uint32_t)((w >> (16 * (lane & 3))) & 0xffffull);
-      c0 = c1 = c2 = 0;
-    };
-    int batches = 0;
-    for (uint32_t q = w0; q < w1; q += 32 * kU) {
-      if (++batches == 256) {
-        flush();
-        batches = 0;
-      }
-      uint32_t d[kU];
-#pragma unroll
-      for (int k = 0; k < kU; ++k) {
-        const uint32_t p = q + 32 * k + lane;
-        d[k] = p < w1 ? dir[p] : 10u;
-      }
-#pragma unroll
-      for (int k = 0; k < kU; ++k) {
-        const unsigned long long one = 1ull << (16 * (d[k] & 3u));
-        if (d[k] < 4u)
-          c0 += one;
-        else if (d[k] < 8u)
-          c1 += one;
-        else if (d[k] < 10u)
-          c2 += one;
-      }
+    for (int u = 0; u < kScatterU; ++u) {
+      const uint32_t p = q + 32 * u + lane;
+      d[u] = p < w1 ? S.dir[p] : 10u;
+      src[u] = p < w1 ? (S.old_order ? S.old_order[p] : S.slot0 + p) : 0u;
     }
-    flush();
-    if (lane < 10) s_cnt[warp][lane] = mycnt;
-    __syncthreads();
-    if (lane < 9) {
-      uint32_t off = grp_off[s * 9 + lane];
-      for (int w = 0; w < warp; ++w) off += s_cnt[w][lane];
-      s_base[warp][lane] = off;
-    }
-    __syncwarp();
-    // pass 2: stable placement
-    uint32_t base4 = s_base[warp][4];
-    for (uint32_t q = w0; q < w1; q += 32 * kU) {
-      uint32_t d[kU], src[kU];
 #pragma unroll
-      for (int k = 0; k < kU; ++k) {
-        const uint32_t p = q + 32 * k + lane;
-        d[k] = p < w1 ? dir[p] : 10u;
-        // no old order (after a compacting push): the particle at list
-        // position p sits in slot slot0 + p
-        src[k] = p < w1 ? (old_order ? old_order[p] : slot0 + p) : 0u;
-      }
-#pragma unroll
-      for (int k = 0; k < kU; ++k) {
-        if (q + 32 * k >= w1) break;
-        const uint32_t dk = d[k];
-        const uint32_t stay = __ballot_sync(0xffffffffu, dk == 4u);
-        const uint32_t other = __ballot_sync(0xffffffffu, dk < 9u && dk != 4u);
-        uint32_t dst = 0xffffffffu;
-        if (dk == 4u) dst = base4 + __popc(stay & lt);
-        base4 += __popc(stay);
-        if (other) {
-          if ((other >> lane) & 1u) {
-            const uint32_t peers = __match_any_sync(other, dk);
-            const uint32_t bs = s_base[warp][dk];
-            dst = bs + __popc(peers & lt);
-            __syncwarp(other);
-            if ((peers & lt) == 0u) s_base[warp][dk] = bs + __popc(peers);
-          }
-          __syncwarp();
+    for (int u = 0; u < kScatterU; ++u) {
+      if (q + 32 * u >= w1) break;
+      const uint32_t dk = d[u];
+      const uint32_t stay = __ballot_sync(0xffffffffu, dk == 4u);
+      const uint32_t other = __ballot_sync(0xffffffffu, dk < 9u && dk != 4u);
+      uint32_t dst = 0xffffffffu;
+      if (dk == 4u) dst = base4 + __popc(stay & lt);
+      base4 += __popc(stay);
+      if (other) {
+        if ((other >> lane) & 1u) {
+          const uint32_t peers = __match_any_sync(other, dk);
+          const uint32_t bs = s_base[dk];
+          dst = bs + __popc(peers & lt);
+          __syncwarp(other);
+          if ((peers & lt) == 0u) s_base[dk] = bs + __popc(peers);
         }
-        if (dst != 0xffffffffu) {
-          if (dst < capacity)
-            new_order[dst] = src[k];
-          else
-            atomicAdd(&status->tile_faults, 1ull);
-        }
+        __syncwarp();
+      }
+      if (dst != 0xffffffffu) {
+        if (dst < S.capacity)
+          S.new_order[dst] = src[u];
+        else
+          atomicAdd(&S.status->tile_faults, 1ull);
       }
     }
-    __syncthreads();
   }
 }
 
-// One pass of the same stable placement, using the per-chunk direction
-// counts the push / deposit kernel recorded (chunk k of source tile s is
-// list entries [k CH, (k + 1) CH) of the tile, its counts at entry
-// old_start[s] / CH + s + k of chunk_count). The CTA turns them into the
-// group offset of every (chunk, direction); warp w then places chunks w,
-// w + 8, ... with the ballot / __match_any_sync ranking of pass 2 above.
-// Tiles of more than kMaxChunks chunks take the two-pass kernel.
+__device__ __forceinline__ void scatter_two_pass(const ScatterOut &S, uint32_t b, uint32_t e,
+                                                 uint32_t (*s_cnt)[10], uint32_t (*s_base)[10],
+                                                 const uint32_t *s_off) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const uint32_t n = e - b;
+  const uint32_t seg = ((n + kScatterWarps * 32 - 1) / (kScatterWarps * 32)) * 32;
+  const uint32_t w0 = b + min(n, warp * seg), w1 = b + min(n, (warp + 1) * seg);
+  // pass 1: direction counts of this warp's segment; packed counters of 16
+  // bits, directions 0-3 in c0, 4-7 in c1, 8-9 in c2, summed over the warp
+  // into lane f's mycnt every 256 batches (at most 32 x 4 x 256 = 32768
+  // entries per counter in between)
+  unsigned long long c0 = 0, c1 = 0, c2 = 0;
+  uint32_t mycnt = 0;  // lane f < 10: count of direction f
+  auto flush = [&]() {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      c0 += __shfl_xor_sync(0xffffffffu, c0, o);
+      c1 += __shfl_xor_sync(0xffffffffu, c1, o);
+      c2 += __shfl_xor_sync(0xffffffffu, c2, o);
+    }
+    const unsigned long long w = lane < 4 ? c0 : (lane < 8 ? c1 : c2);
+    if (lane < 10) mycnt += (uint32_t)((w >> (16 * (lane & 3))) & 0xffffull);
+    c0 = c1 = c2 = 0;
+  };
+  int batches = 0;
+  for (uint32_t q = w0; q < w1; q += 32 * kScatterU) {
+    if (++batches == 256) {
+      flush();
+      batches = 0;
+    }
+    uint32_t d[kScatterU];
+#pragma unroll
+    for (int k = 0; k < kScatterU; ++k) {
+      const uint32_t p = q + 32 * k + lane;
+      d[k] = p < w1 ? S.dir[p] : 10u;
+    }
+#pragma unroll
+    for (int k = 0; k < kScatterU; ++k) {
+      const unsigned long long one = 1ull << (16 * (d[k] & 3u));
+      if (d[k] < 4u)
+        c0 += one;
+      else if (d[k] < 8u)
+        c1 += one;
+      else if (d[k] < 10u)
+        c2 += one;
+    }
+  }
+  flush();
+  if (lane < 10) s_cnt[warp][lane] = mycnt;
+  __syncthreads();
+  if (lane < 9) {
+    uint32_t off = s_off[lane];
+    for (int w = 0; w < warp; ++w) off += s_cnt[w][lane];
+    s_base[warp][lane] = off;
+  }
+  __syncwarp();
+  // pass 2: stable placement
+  scatter_walk(S, w0, w1, s_base[warp]);
+}
+
+// One CTA per source tile. With the per-chunk direction counts the push /
+// deposit kernel recorded (chunk k of source tile s is list entries [k CH,
+// (k + 1) CH) of the tile, its counts at entry old_start[s] / CH + s + k of
+// chunk_count) the placement takes one pass: the counts become the group
+// offset of every (chunk, direction), and warp w places chunks w, w + 8, ...
+// Without them, and for tiles of more than kMaxChunks chunks, two passes.
 constexpr int kMaxChunks = 128;
 
 __global__ void __launch_bounds__(kScatterThreads)
-    k_order_scatter1(int ntiles, int ch, const uint32_t *__restrict__ old_start,
-                     const uint32_t *__restrict__ old_order, const uint8_t *__restrict__ dir,
-                     const uint32_t *__restrict__ chunk_count, const uint32_t *__restrict__ grp_off,
-                     uint32_t *__restrict__ new_order, uint32_t capacity, uint32_t slot0,
-                     uint32_t *__restrict__ big_tiles, DevStatus *status) {
-  constexpr int kWarps = kScatterThreads / 32;
-  constexpr int kU = 4;
+    k_order_scatter(int ntiles, int ch, const uint32_t *__restrict__ old_start,
+                    const uint32_t *__restrict__ grp_off,
+                    const uint32_t *__restrict__ chunk_count, ScatterOut S) {
   __shared__ uint32_t s_cb[kMaxChunks][9];  // group offset of each (chunk, direction)
-  __shared__ uint32_t s_base[kWarps][9];
+  __shared__ uint32_t s_base[kScatterWarps][10];
+  __shared__ uint32_t s_cnt[kScatterWarps][10];
+  __shared__ uint32_t s_off[9];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const uint32_t lt = (1u << lane) - 1u;
   for (int s = blockIdx.x; s < ntiles; s += gridDim.x) {
     const uint32_t b = old_start[s], e = old_start[s + 1];
     const uint32_t n = e - b;
     const int nch = (int)((n + ch - 1) / ch);
-    if (nch > kMaxChunks) {  // left to the two-pass kernel
-      if (tid == 0) big_tiles[1 + atomicAdd(big_tiles, 1u)] = (uint32_t)s;
-      continue;
-    }
-    const size_t c0 = (size_t)(b / ch) + s;
-    // the tile's chunk counts, loaded by all threads, then scanned per
-    // direction in shared memory
-    for (int i = tid; i < nch * 9; i += kScatterThreads)
-      s_cb[i / 9][i % 9] = chunk_count[(c0 + i / 9) * 10 + i % 9];
     const uint32_t off = tid < 9 ? grp_off[s * 9 + tid] : 0u;
-    __syncthreads();
-    if (tid < 9) {
-      uint32_t run = off;
-      for (int k = 0; k < nch; ++k) {
-        const uint32_t v = s_cb[k][tid];
-        s_cb[k][tid] = run;
-        run += v;
-      }
-    }
-    __syncthreads();
-    for (int k = warp; k < nch; k += kWarps) {
-      if (lane < 9) s_base[warp][lane] = s_cb[k][lane];
-      __syncwarp();
-      uint32_t base4 = s_base[warp][4];
-      const uint32_t w0 = b + (uint32_t)k * ch, w1 = min(e, w0 + ch);
-      for (uint32_t q = w0; q < w1; q += 32 * kU) {
-        uint32_t d[kU], src[kU];
-#pragma unroll
-        for (int u = 0; u < kU; ++u) {
-          const uint32_t p = q + 32 * u + lane;
-          d[u] = p < w1 ? dir[p] : 10u;
-          src[u] = p < w1 ? (old_order ? old_order[p] : slot0 + p) : 0u;
-        }
-#pragma unroll
-        for (int u = 0; u < kU; ++u) {
-          if (q + 32 * u >= w1) break;
-          const uint32_t dk = d[u];
-          const uint32_t stay = __ballot_sync(0xffffffffu, dk == 4u);
-          const uint32_t other = __ballot_sync(0xffffffffu, dk < 9u && dk != 4u);
-          uint32_t dst = 0xffffffffu;
-          if (dk == 4u) dst = base4 + __popc(stay & lt);
-          base4 += __popc(stay);
-          if (other) {
-            if ((other >> lane) & 1u) {
-              const uint32_t peers = __match_any_sync(other, dk);
-              const uint32_t bs = s_base[warp][dk];
-              dst = bs + __popc(peers & lt);
-              __syncwarp(other);
-              if ((peers & lt) == 0u) s_base[warp][dk] = bs + __popc(peers);
-            }
-            __syncwarp();
-          }
-          if (dst != 0xffffffffu) {
-            if (dst < capacity)
-              new_order[dst] = src[u];
-            else
-              atomicAdd(&status->tile_faults, 1ull);
-          }
+    if (chunk_count && nch <= kMaxChunks) {
+      const size_t c0 = (size_t)(b / ch) + s;
+      // the tile's chunk counts, loaded by all threads, then scanned per
+      // direction in shared memory
+      for (int i = tid; i < nch * 9; i += kScatterThreads)
+        s_cb[i / 9][i % 9] = chunk_count[(c0 + i / 9) * 10 + i % 9];
+      __syncthreads();
+      if (tid < 9) {
+        uint32_t run = off;
+        for (int k = 0; k < nch; ++k) {
+          const uint32_t v = s_cb[k][tid];
+          s_cb[k][tid] = run;
+          run += v;
         }
       }
-      __syncwarp();
+      __syncthreads();
+      for (int k = warp; k < nch; k += kScatterWarps) {
+        if (lane < 9) s_base[warp][lane] = s_cb[k][lane];
+        __syncwarp();
+        const uint32_t w0 = b + (uint32_t)k * ch, w1 = min(e, w0 + ch);
+        scatter_walk(S, w0, w1, s_base[warp]);
+        __syncwarp();
+      }
+    } else {
+      if (tid < 9) s_off[tid] = off;  // read after the barrier between the passes
+      scatter_two_pass(S, b, e, s_cnt, s_base, s_off);
     }
     __syncthreads();
   }
 }
 
 // start[k] = first position of key k in the sorted keys[0, n), for
-// k = 0..nbins (start[nbins] = position of the first key >= nbins); also the
-// largest segment length over keys < nbins.
+// k = 0..nbins (start[nbins] = position of the first key >= nbins).
+// Four consecutive keys per thread and round (one 16-byte load of the aligned
+// keys and the key before them): one key per thread and round was bound by the
+// latency of its loads (26 us for 8.4 M keys, 33 MB).
 __global__ void k_segment_starts(const uint32_t *__restrict__ keys, size_t n, uint32_t nbins,
                                  uint32_t *__restrict__ start) {
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i <= n;
-       i += (size_t)gridDim.x * blockDim.x) {
-    const uint32_t prev = (i == 0) ? 0u : min(keys[i - 1], nbins) + 1u;  // first key not yet started
-    const uint32_t cur = (i == n) ? nbins : min(keys[i], nbins);
-    for (uint32_t k = prev; k <= cur; ++k) start[k] = (uint32_t)i;
+  for (size_t i0 = (blockIdx.x * (size_t)blockDim.x + threadIdx.x) * 4; i0 <= n;
+       i0 += (size_t)gridDim.x * blockDim.x * 4) {
+    uint32_t k[4];
+    if (i0 + 3 < n) {
+      const uint4 q = *reinterpret_cast<const uint4 *>(keys + i0);
+      k[0] = q.x;
+      k[1] = q.y;
+      k[2] = q.z;
+      k[3] = q.w;
+    } else {
+#pragma unroll
+      for (int u = 0; u < 4; ++u) k[u] = i0 + u < n ? keys[i0 + u] : nbins;
+    }
+    uint32_t prev = i0 == 0 ? 0u : min(keys[i0 - 1], nbins) + 1u;  // first key not yet started
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const uint32_t cur = min(k[u], nbins);
+      if (i0 + u <= n)
+        for (; prev <= cur; ++prev) start[prev] = (uint32_t)(i0 + u);
+    }
   }
-}
-
-__global__ void __launch_bounds__(kScanThreads)
-    k_segment_max(const uint32_t *__restrict__ start, uint32_t nbins, uint32_t *n_max) {
-  __shared__ uint32_t s_max;
-  if (threadIdx.x == 0) s_max = 0;
-  __syncthreads();
-  uint32_t mx = 0;
-  for (uint32_t k = threadIdx.x; k < nbins; k += blockDim.x) mx = max(mx, start[k + 1] - start[k]);
-  atomicMax(&s_max, mx);
-  __syncthreads();
-  if (threadIdx.x == 0) *n_max = s_max;
 }
 
 // Tile order of particles sorted by cell: the particles of tile t are, row
@@ -417,38 +386,103 @@ __global__ void k_tile_keys(MeshK m, TilesK T, uint32_t *cell, size_t base, size
   }
 }
 
-// Exclusive scan of nbins counters into start[0..nbins] with one CTA.
-__global__ void __launch_bounds__(kScanThreads)
-    k_scan_counts(const uint32_t *counts, int nbins, uint32_t *start, uint32_t *n_max) {
-  __shared__ uint32_t s_part[kScanThreads];
-  __shared__ uint32_t s_max;
-  const int tid = threadIdx.x;
-  if (tid == 0) s_max = 0;
-  const int per = (nbins + kScanThreads - 1) / kScanThreads;
-  const int b0 = tid * per, b1 = min(nbins, b0 + per);
-  uint32_t local = 0, mx = 0;
-  for (int b = b0; b < b1; ++b) {
-    local += counts[b];
-    mx = max(mx, counts[b]);
+// Exclusive scan of nbins tile populations into start[0..nbins] with one CTA,
+// four consecutive tiles per thread and 4096 per round with a carry (coalesced
+// 16-byte loads; one thread per contiguous run of counters took 22 us on
+// 16384 tiles, bound by its strided loads); the largest population goes to
+// n_max[0]. With kPop the populations are the new ones, computed here (up to
+// 1024 tiles, one per thread); with kStarts they are the differences of a
+// start array that stands already.
+// The same pass lists the push / deposit's work items: a tile of n particles
+// gives ceil(n / item_len) of them, their number in n_max[1], item_len in
+// n_max[2].
+enum ScanSource { kCounts, kPop, kStarts };
+
+struct ItemOut {
+  uint2 *items;
+  uint32_t cap, len;
+};
+
+__device__ __forceinline__ uint32_t warp_scan(uint32_t v, int lane) {
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t t = __shfl_up_sync(0xffffffffu, v, o);
+    if (lane >= o) v += t;
   }
-  s_part[tid] = local;
-  __syncthreads();
-  atomicMax(&s_max, mx);
-  for (int off = 1; off < kScanThreads; off <<= 1) {
-    uint32_t v = tid >= off ? s_part[tid - off] : 0u;
-    __syncthreads();
-    s_part[tid] += v;
-    __syncthreads();
-  }
-  uint32_t run = s_part[tid] - local;
-  for (int b = b0; b < b1; ++b) {
-    start[b] = run;
-    run += counts[b];
-  }
-  if (tid == kScanThreads - 1) start[nbins] = s_part[tid];
-  __syncthreads();
-  if (tid == 0 && n_max) *n_max = s_max;
+  return v;
 }
+
+template <ScanSource kSrc>
+__global__ void __launch_bounds__(kScanThreads)
+    k_scan_counts(TileTopo T, const uint32_t *__restrict__ counts, int nbins,
+                  uint32_t *start, uint32_t *n_max, ItemOut I, uint32_t *__restrict__ grp_off) {
+  constexpr int kPer = kSrc == kCounts ? 4 : 1;
+  __shared__ uint32_t s_w[kScanThreads / 32], s_i[kScanThreads / 32];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  uint32_t carry = 0, icarry = 0, mx = 0;
+  for (int b0 = 0; b0 < nbins; b0 += kPer * kScanThreads) {
+    const int b = b0 + tid * kPer;
+    uint32_t v[kPer];
+    if constexpr (kSrc == kPop) {
+      v[0] = b < nbins ? new_population(T, counts, b) : 0u;
+    } else if constexpr (kSrc == kStarts) {
+      v[0] = b < nbins ? counts[b + 1] - counts[b] : 0u;
+    } else if (b + 3 < nbins) {
+      const uint4 q = *reinterpret_cast<const uint4 *>(counts + b);
+      v[0] = q.x;
+      v[1] = q.y;
+      v[2] = q.z;
+      v[3] = q.w;
+    } else {
+#pragma unroll
+      for (int k = 0; k < kPer; ++k) v[k] = b + k < nbins ? counts[b + k] : 0u;
+    }
+    uint32_t own = 0, iown = 0;
+#pragma unroll
+    for (int k = 0; k < kPer; ++k) {
+      own += v[k];
+      iown += (v[k] + I.len - 1) / I.len;
+      mx = max(mx, v[k]);
+    }
+    const uint32_t inc = warp_scan(own, lane), iinc = warp_scan(iown, lane);
+    if (lane == 31) {
+      s_w[warp] = inc;
+      s_i[warp] = iinc;
+    }
+    __syncthreads();
+    // every warp scans the warp sums
+    const uint32_t ws = warp_scan(s_w[lane], lane), is = warp_scan(s_i[lane], lane);
+    const uint32_t before = __shfl_sync(0xffffffffu, ws, max(warp - 1, 0));
+    const uint32_t ibefore = __shfl_sync(0xffffffffu, is, max(warp - 1, 0));
+    uint32_t run = carry + (warp ? before : 0u) + inc - own;
+    uint32_t item = icarry + (warp ? ibefore : 0u) + iinc - iown;
+#pragma unroll
+    for (int k = 0; k < kPer; ++k) {
+      if (kSrc != kStarts && b + k < nbins) start[b + k] = run;
+      run += v[k];
+      for (uint32_t p = 0; p < v[k]; p += I.len, ++item)
+        if (item < I.cap) I.items[item] = make_uint2((uint32_t)(b + k), p);
+    }
+    carry += __shfl_sync(0xffffffffu, ws, 31);
+    icarry += __shfl_sync(0xffffffffu, is, 31);
+    __syncthreads();
+  }
+  if (kSrc != kStarts && tid == 0) start[nbins] = carry;
+  if (kSrc == kPop && grp_off && tid < nbins * 9)  // the barrier above: start stands
+    grp_off[tid] = group_offset(T, counts, start, tid / 9, tid % 9);
+  mx = __reduce_max_sync(0xffffffffu, mx);
+  if (lane == 0) s_w[warp] = mx;
+  __syncthreads();
+  if (warp == 0) {
+    mx = __reduce_max_sync(0xffffffffu, s_w[lane]);
+    if (lane == 0) {
+      n_max[0] = mx;
+      n_max[1] = min(icarry, I.cap);
+      n_max[2] = I.len;
+    }
+  }
+}
+static_assert(kScanThreads == 1024, "one warp scans the 32 warp sums");
 
 // Keys of slots base + i, i < n (vals = the slots); slots at or beyond a
 // device-side live count are empty.
@@ -492,41 +526,61 @@ cudaError_t radix_pairs(Ctx &c, size_t n, int end_bit, uint32_t **keys_out,
 
 }  // namespace
 
+namespace {
+
+TileTopo topo_of(const Ctx &c) {
+  return TileTopo{c.tiles.ntx, c.tiles.nty, c.tiles.ntiles, c.params.periodic[0],
+                  c.params.periodic[1]};
+}
+
+// Work items of the next push: about three per resident CTA (four per SM), so
+// that neither a grid of few tiles nor a few crowded tiles leave the rest of
+// the chip idle at the end; a tile of at most one item's length stays whole.
+// An item costs its field tile, a cleared and a flushed current tile, about
+// 2 us beside the 3 - 6 us of a 256-particle chunk.
+ItemOut item_out(Ctx &c) {
+  const uint32_t ch = (uint32_t)chunk_of(c);
+  const size_t n = c.item_total > 0 ? c.item_total : c.number - c.store_base;
+  const size_t slots = (size_t)c.num_sms * 4 * 3;
+  const size_t chunks = (n / ch + slots - 1) / slots;
+  c.item_len = ch * (uint32_t)(chunks < 1 ? 1 : chunks);
+  return ItemOut{c.items, (uint32_t)c.items_cap, c.item_len};
+}
+
+}  // namespace
+
 cudaError_t launch_tile_scan(Ctx &c, const uint32_t *dir_count, uint32_t *new_start,
                              uint32_t *grp_off) {
-  TileTopo T{c.tiles.ntx, c.tiles.nty, c.tiles.ntiles, c.params.periodic[0],
-             c.params.periodic[1]};
+  const TileTopo T = topo_of(c);
   const int nt = c.tiles.ntiles;
-  const int g = (nt + 255) / 256;
-  k_tile_newcount<<<g, 256, 0, c.stream>>>(T, dir_count, c.newcount);
-  k_scan_counts<<<1, kScanThreads, 0, c.stream>>>(c.newcount, nt, new_start, c.n_max);
-  k_tile_groups<<<g, 256, 0, c.stream>>>(T, dir_count, new_start, grp_off);
-  c.launches += 3;
+  const ItemOut I = item_out(c);
+  const bool groups = nt * 9 <= kScanThreads;  // in the scan's block
+  if (nt <= kScanThreads) {
+    k_scan_counts<kPop><<<1, kScanThreads, 0, c.stream>>>(T, dir_count, nt, new_start, c.n_max, I,
+                                                          groups ? grp_off : nullptr);
+    c.launches++;
+  } else {
+    k_tile_newcount<<<(nt + 127) / 128, 128, 0, c.stream>>>(T, dir_count, c.newcount);
+    k_scan_counts<kCounts><<<1, kScanThreads, 0, c.stream>>>(T, c.newcount, nt, new_start,
+                                                             c.n_max, I, nullptr);
+    c.launches += 2;
+  }
+  if (!groups) {
+    k_tile_groups<<<(nt * 9 + 255) / 256, 256, 0, c.stream>>>(T, dir_count, new_start, grp_off);
+    c.launches++;
+  }
   return cudaGetLastError();
 }
 
 cudaError_t launch_order_scatter(Ctx &c, const uint32_t *old_start, const uint32_t *old_order,
                                  const uint8_t *dir, const uint32_t *grp_off,
                                  uint32_t *new_order, uint32_t slot0) {
-  int grid = c.tiles.ntiles < c.num_sms * 8 ? c.tiles.ntiles : c.num_sms * 8;
-  if (!c.chunk_count_ok) {
-    k_order_scatter<<<grid, kScatterThreads, 0, c.stream>>>(
-        c.tiles.ntiles, old_start, old_order, dir, grp_off, new_order, (uint32_t)c.order_cap,
-        slot0, nullptr, c.status);
-    c.launches++;
-    return cudaGetLastError();
-  }
-  // one pass from the push / deposit kernel's chunk counts; tiles of more
-  // than kMaxChunks chunks are listed in big_tiles for the two-pass kernel
-  cudaError_t e = cudaMemsetAsync(c.big_tiles, 0, sizeof(uint32_t), c.stream);
-  if (e != cudaSuccess) return e;
-  k_order_scatter1<<<grid, kScatterThreads, 0, c.stream>>>(
-      c.tiles.ntiles, chunk_of(c), old_start, old_order, dir, c.chunk_count, grp_off, new_order,
-      (uint32_t)c.order_cap, slot0, c.big_tiles, c.status);
-  k_order_scatter<<<c.num_sms, kScatterThreads, 0, c.stream>>>(
-      c.tiles.ntiles, old_start, old_order, dir, grp_off, new_order, (uint32_t)c.order_cap,
-      slot0, c.big_tiles, c.status);
-  c.launches += 2;
+  const int grid = c.tiles.ntiles < c.num_sms * 8 ? c.tiles.ntiles : c.num_sms * 8;
+  const ScatterOut S{old_order, dir, new_order, (uint32_t)c.order_cap, slot0, c.status};
+  k_order_scatter<<<grid, kScatterThreads, 0, c.stream>>>(
+      c.tiles.ntiles, chunk_of(c), old_start, grp_off,
+      c.chunk_count_ok ? c.chunk_count : nullptr, S);
+  c.launches++;
   return cudaGetLastError();
 }
 
@@ -684,13 +738,15 @@ cudaError_t rebuild_tile_order(Ctx &c) {
     e = cudaMemcpyAsync(c.order[c.cur], vo, n * sizeof(uint32_t), cudaMemcpyDeviceToDevice,
                         c.stream);
     if (e != cudaSuccess) return e;
-    k_segment_starts<<<grid_for(c, n + 1, 256), 256, 0, c.stream>>>(ko, n, nt, start);
+    k_segment_starts<<<grid_for(c, n / 4 + 1, 256), 256, 0, c.stream>>>(ko, n, nt, start);
     c.launches++;
   } else {
     e = cudaMemsetAsync(start, 0, sizeof(uint32_t) * (nt + 1), c.stream);
     if (e != cudaSuccess) return e;
   }
-  k_segment_max<<<1, kScanThreads, 0, c.stream>>>(start, nt, c.n_max);
+  const ItemOut I = item_out(c);
+  k_scan_counts<kStarts><<<1, kScanThreads, 0, c.stream>>>(topo_of(c), start, (int)nt, nullptr,
+                                                           c.n_max, I, nullptr);
   c.launches++;
   c.order_valid = true;
   return cudaGetLastError();
@@ -705,7 +761,9 @@ cudaError_t tile_order_from_cells(Ctx &c, uint32_t slot0) {
   const int nt = c.tiles.ntiles;
   k_tile_counts_from_cells<<<(nt + 255) / 256, 256, 0, c.stream>>>(c.mk, c.tiles, c.cell_start,
                                                                    c.dir_count);
-  k_scan_counts<<<1, kScanThreads, 0, c.stream>>>(c.dir_count, nt, c.tile_start[c.cur], c.n_max);
+  k_scan_counts<kCounts><<<1, kScanThreads, 0, c.stream>>>(topo_of(c), c.dir_count, nt,
+                                                           c.tile_start[c.cur], c.n_max,
+                                                           item_out(c), nullptr);
   k_tile_fill_from_cells<<<nt < c.num_sms * 8 ? nt : c.num_sms * 8, 256, 0, c.stream>>>(
       c.mk, c.tiles, c.cell_start, c.tile_start[c.cur], c.order[c.cur], slot0);
   c.launches += 3;
@@ -791,7 +849,7 @@ cudaError_t sort_by_cell(Ctx &c, size_t *new_number) {
     e = cudaMalloc(&c.cell_start, sizeof(uint32_t) * ((size_t)ncells + 1));
     if (e != cudaSuccess) return e;
   }
-  k_segment_starts<<<grid_for(c, n + 1, 256), 256, 0, c.stream>>>(ko, n, ncells, c.cell_start);
+  k_segment_starts<<<grid_for(c, n / 4 + 1, 256), 256, 0, c.stream>>>(ko, n, ncells, c.cell_start);
   c.launches++;
   if (device_count) {
     c.number_stale = true;
@@ -857,7 +915,7 @@ cudaError_t sort_photons(Ctx &c, size_t *new_number) {
     e = cudaMalloc(&c.cell_start, sizeof(uint32_t) * ((size_t)ncells + 1));
     if (e != cudaSuccess) return e;
   }
-  k_segment_starts<<<grid_for(c, n + 1, 256), 256, 0, c.stream>>>(ko, n, ncells, c.cell_start);
+  k_segment_starts<<<grid_for(c, n / 4 + 1, 256), 256, 0, c.stream>>>(ko, n, ncells, c.cell_start);
   c.launches++;
   uint32_t live = 0;
   e = cudaMemcpyAsync(&live, c.cell_start + ncells, sizeof(uint32_t), cudaMemcpyDeviceToHost,
