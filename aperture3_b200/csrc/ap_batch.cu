@@ -33,15 +33,15 @@ struct Group {
   std::vector<int> members;  // indices into the batch's runs
 };
 
-// Work items of a run in a batched launch: tiles (2D) or chunks of
-// particle slots (1D).
+// Work items of a run in a batched launch: chunks of particle slots (1D), or
+// at most this many parts of tile lists (2D; the lists stand on the device).
 uint32_t work_items(const Ctx *c) {
   if (c->mk.dim == 1) {
     // with a device-side count the kernel covers the capacity
     const size_t n = c->pstate ? c->capacity : c->number;
     return (uint32_t)((n + kChunk1DSlots - 1) / kChunk1DSlots);
   }
-  return (uint32_t)c->tiles.ntiles;
+  return (uint32_t)(c->tiles.ntiles + (c->number - c->store_base) / c->item_len);
 }
 
 }  // namespace
@@ -254,7 +254,7 @@ int launch_groups(ap_batch *b, const std::vector<Group> &gs,
                         sizeof(uint32_t) * kb, cudaMemcpyHostToDevice, b->stream));
   if (!b->capture) B_TRY(cudaEventRecord(b->stage_ev[s], b->stream));
   const RunDesc *dd = reinterpret_cast<const RunDesc *>(dblk);
-  const uint32_t *db = reinterpret_cast<const uint32_t *>(dblk + sizeof(RunDesc) * nr);
+  uint32_t *db = reinterpret_cast<uint32_t *>(dblk + sizeof(RunDesc) * nr);
   for (size_t gi = 0; gi < gs.size(); ++gi) {
     const Group &g = gs[gi];
     if (g.dim == 1)
@@ -278,6 +278,11 @@ int batch_update(ap_batch *b, const double *dt, const uint32_t *steps) {
   std::vector<PushDepositParams> P(n);
   std::vector<bool> work(n, false);
   bool do_rho = false;
+  // the runs of a launch share its blocks, so their work items have one length
+  size_t total = 0;
+  for (const Ctx *c : b->runs)
+    if (c->mk.dim == 2) total += c->number - c->store_base;
+  for (Ctx *c : b->runs) c->item_total = total;
   // 1D runs: accumulator clearing and finalize are batched launches
   std::vector<Run1D> d1;
   std::vector<uint32_t> zero_items, fin_items;
@@ -419,6 +424,7 @@ AP_API int ap_batch_remove(ap_batch *b, ap_ctx *c) {
   if (it == b->runs.end()) return AP_ERR_INVALID;
   B_TRY(cudaStreamSynchronize(b->stream));
   b->runs.erase(it);
+  c->item_total = 0;
   // the run goes back to synchronous calls on the default stream
   ap_set_stream(c, nullptr);
   c->sync = true;
@@ -438,6 +444,7 @@ AP_API int ap_batch_destroy(ap_batch *b) {
   for (Ctx *c : b->runs) {
     ap_set_stream(static_cast<ap_ctx *>(c), nullptr);
     c->sync = true;
+    c->item_total = 0;
   }
   release(b);
   delete b;

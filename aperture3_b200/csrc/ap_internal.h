@@ -460,11 +460,12 @@ constexpr size_t kControlHead = 64;  // bytes before the direction counts
 
 // One persistent push / deposit launch over the tiles of several 2D
 // Cartesian runs with the same tile shape, chunk and field-load path.
-// runs / base are device arrays (base has nruns + 1 entries).
+// runs / base are device arrays; base (nruns + 1 entries) is written here, from
+// the runs' item counts on the device. total: about how many items there are.
 cudaError_t launch_push_deposit_2d_batch(cudaStream_t stream, int num_sms, int tx, int ty,
                                          int chunk, bool tma, bool do_rho, int max_species,
-                                         const RunDesc *runs, const uint32_t *base, int nruns,
-                                         uint32_t total_tiles, uint32_t *queue);
+                                         const RunDesc *runs, uint32_t *base, int nruns,
+                                         uint32_t total, uint32_t *queue);
 // The same for 1D runs: work items are chunks of 2048 particle slots
 // (base[r] = first chunk of run r).
 cudaError_t launch_push_deposit_1d_batch(cudaStream_t stream, int num_sms, bool do_rho,

@@ -166,6 +166,9 @@ struct TileGeom {
   static constexpr int BX = TX + 8;   // field box width: x start rounded down to 4 floats
   static constexpr int BY = TY + 2;   // one halo row on each side
   static constexpr int FSZ = ((BX * BY + 31) / 32) * 32;  // 128-byte aligned stride
+  static constexpr size_t raw_bytes() { return 4 * 6 * FSZ; }  // the six loaded components
+  static constexpr int RX = TX + 1;   // field records of nodes x0 - 1 .. x0 + TX - 1 of a row
+  static constexpr size_t rec_bytes() { return (48 * RX * BY + 127) / 128 * 128; }
   static constexpr int JX = TX + 4;   // J tile: two halo cells on each side
   static constexpr int JY = TY + 4;
   static constexpr int JSZ = JX * JY;
@@ -175,9 +178,15 @@ struct TileGeom {
   static constexpr int NBUF = pipelined<CH>() ? 2 : 1;
   // double-buffered chunks: the order indices of the next two chunks
   static constexpr size_t order_bytes() { return NBUF == 2 ? 2 * 4 * CH : 0; }
+  // the components land in the last staged-chunk buffer, which the first
+  // chunk of an item does not use when there are two
+  static constexpr size_t stage0_bytes() { return NBUF == 2 ? (stage_bytes() + 127) / 128 * 128 : 0; }
+  static constexpr size_t stage1_bytes() {
+    return stage_bytes() > raw_bytes() ? stage_bytes() : raw_bytes();
+  }
   static size_t smem_bytes(int nrho, bool ls = false) {
-    return HDR + 4 * 6 * FSZ + 8 * (3 + nrho) * JSZ + NBUF * stage_bytes() + (ls ? 4 * JSZ : 0) +
-           order_bytes();
+    return HDR + rec_bytes() + stage0_bytes() + stage1_bytes() + 8 * (3 + nrho) * JSZ +
+           (ls ? 4 * JSZ : 0) + order_bytes();
   }
 };
 
@@ -205,8 +214,8 @@ __device__ __forceinline__ uint32_t *param_smem() {
 // The fused push + deposit over the tiles of one run (kMulti false: the
 // parameters P0 and tensor maps maps0 live in the kernel's parameter
 // space) or of a batch of runs (kMulti true: runs[r] in global memory,
-// run r owning tiles [base[r], base[r + 1]) of one queue; each CTA copies
-// the parameters of the run whose tile it takes into shared memory, so
+// run r owning items [base[r], base[r + 1]) of one queue; each CTA copies
+// the parameters of the run whose item it takes into shared memory, so
 // the per-particle code reads them from there and not through global
 // loads that the particle stores could alias).
 template <int TX, int TY, int CH, bool kTMA, bool kRho, bool kLS, bool kMulti>
@@ -223,7 +232,16 @@ __device__ __forceinline__ void push_deposit_tiles(const PushDepositParams &P0,
   int *s_tile = reinterpret_cast<int *>(smem + 8);
   int *s_abort = reinterpret_cast<int *>(smem + 12);
   uint32_t *s_cnt = reinterpret_cast<uint32_t *>(smem + 16);
-  float *sF = reinterpret_cast<float *>(smem + G::HDR);
+  // field records of the tile's nodes (i, j): pairs of nodes i, i + 1, so that
+  // a particle reads the four nodes of a component as two aligned vectors:
+  // sEB[0] = (E1, E1+, B2, B2+), sEB[1] = (E2, E2+, B1, B1+) (the two
+  // components of one record share their stagger), sZ[0] = (E3, E3+),
+  // sZ[1] = (B3, B3+)
+  constexpr int kNodes = G::RX * G::BY;
+  float4 *sEB = reinterpret_cast<float4 *>(smem + G::HDR);
+  float2 *sZ = reinterpret_cast<float2 *>(sEB + 2 * kNodes);
+  unsigned char *s_stage = smem + G::HDR + G::rec_bytes();
+  float *sRaw = reinterpret_cast<float *>(s_stage + G::stage0_bytes());
   const int tid = threadIdx.x;
   const int lane = tid & 31, warp = tid >> 5;
 
@@ -241,8 +259,9 @@ __device__ __forceinline__ void push_deposit_tiles(const PushDepositParams &P0,
     __syncthreads();
     const int g = *s_tile;
     const CUtensorMap *mp = maps0;
-    int t = g;
-    uint32_t item0 = 0;  // this work item's first list entry of the tile
+    const uint32_t *n_items = P0.n_items;
+    const uint2 *items = P0.items;
+    int k = g;  // work item of the run
     if constexpr (kMulti) {
       if ((uint32_t)g >= base[nruns]) break;
       int lo = 0, hi = nruns - 1;  // largest r with base[r] <= g
@@ -256,25 +275,26 @@ __device__ __forceinline__ void push_deposit_tiles(const PushDepositParams &P0,
         s_pbuf[i] = src[i];
       __syncthreads();
       mp = runs[lo].maps.m;
-      t = g - (int)base[lo];
+      k = g - (int)base[lo];
+      n_items = reinterpret_cast<const PushDepositParams *>(s_pbuf)->n_items;
+      items = reinterpret_cast<const PushDepositParams *>(s_pbuf)->items;
     } else {
-      if ((uint32_t)g >= *P0.n_items) break;
-      const uint2 it = P0.items[g];
-      t = (int)it.x;
-      item0 = it.y;
+      if ((uint32_t)k >= *n_items) break;
     }
+    const uint2 item = items[k];
+    const int t = (int)item.x;  // its tile, and the first and last list entry
+    const int p0 = (int)item.y;
+    const uint32_t item_len = n_items[1];
     const PushDepositParams &P =
         kMulti ? *reinterpret_cast<const PushDepositParams *>(s_pbuf) : P0;
 
     // shared-memory layout of this run (the charge tile depends on its
     // number of species)
     const int ncomp = 3 + (kRho ? P.num_species : 0);
-    int *sJhi = reinterpret_cast<int *>(sF + 6 * G::FSZ);
+    int *sJhi = reinterpret_cast<int *>(s_stage + G::stage0_bytes() + G::stage1_bytes());
     unsigned *sJlo = reinterpret_cast<unsigned *>(sJhi + ncomp * G::JSZ);
-    float *st = reinterpret_cast<float *>(sJlo + ncomp * G::JSZ);
     // log-spherical: cell volumes over the J tile window
-    float *s_dv = reinterpret_cast<float *>(reinterpret_cast<unsigned char *>(st) +
-                                            G::NBUF * G::stage_bytes());
+    float *s_dv = reinterpret_cast<float *>(sJlo + ncomp * G::JSZ);
     uint32_t *s_ord = reinterpret_cast<uint32_t *>(s_dv + (kLS ? G::JSZ : 0));
     const int dims0 = P.m.dims[0], dims1 = P.m.dims[1];
     const int g0 = P.m.guard[0], g1 = P.m.guard[1];
@@ -284,7 +304,7 @@ __device__ __forceinline__ void push_deposit_tiles(const PushDepositParams &P0,
     const int lg = max(4, bits_of(*P.n_max));
     const FixedFmt fx = fixed_format(lg, 63 - 2 * lg, P.qmax * *P.wmax);
     const float fscale = ldexpf(1.0f, fx.S);
-    if ((kMulti ? t : g) == 0 && tid == 0) *P.fx_used = fx;
+    if (k == 0 && tid == 0) *P.fx_used = fx;
 
     const int tix = t % P.t.ntx, tiy = t / P.t.ntx;
     const int x0 = g0 + tix * TX, y0 = g1 + tiy * TY;
@@ -296,8 +316,7 @@ __device__ __forceinline__ void push_deposit_tiles(const PushDepositParams &P0,
     // the gathers of the next chunk never wait for them
     const uint32_t base = P.tile_start[t];
     const int n_tile = (int)(P.tile_start[t + 1] - base);
-    const int p0 = (int)item0;
-    const int n_t = kMulti ? n_tile : min(n_tile, p0 + (int)P.n_items[1]);  // end of the item
+    const int n_t = min(n_tile, p0 + (int)item_len);  // end of the item
     auto prefetch_order = [&](int c0) {
       uint32_t *dst = s_ord + ((c0 / CH) & 1) * CH;
       const int nch = min(CH, n_t - c0);
@@ -309,52 +328,9 @@ __device__ __forceinline__ void push_deposit_tiles(const PushDepositParams &P0,
       if (p0 + CH < n_t) prefetch_order(p0 + CH);
     }
 
-    // 1. field tile
-    if (kTMA) {
-      if (tid == 0) {
-        fence_proxy_async_smem();
-        mbar_expect_tx(mbar, 6u * G::BX * G::BY * 4u);
-#pragma unroll
-        for (int k = 0; k < 6; ++k) tma_load_2d(sF + k * G::FSZ, mp + k, xs, ys, mbar);
-      }
-    } else {
-      for (int i = tid; i < 6 * G::BX * G::BY; i += kThreads2D) {
-        int k = i / (G::BX * G::BY), rem = i % (G::BX * G::BY);
-        int yy = ys + rem / G::BX, xx = xs + rem % G::BX;
-        float v = 0.0f;
-        if (xx < dims0 && yy < dims1) v = P.F[k].ptr[(size_t)yy * P.F[k].pitch + xx];
-        sF[k * G::FSZ + rem] = v;
-      }
-    }
-    // 2. zero the current (and charge) tile
-    for (int i = tid; i < nacc; i += kThreads2D) {
-      sJhi[i] = 0;
-      sJlo[i] = 0u;
-    }
-    if constexpr (kLS) {
-      for (int i = tid; i < G::JSZ; i += kThreads2D) {
-        const int gx = jx0 + i % G::JX, gy = jy0 + i / G::JX;
-        s_dv[i] = (gx < dims0 && gy < dims1) ? P.dV.ptr[(size_t)gy * P.dV.pitch + gx] : 1.0f;
-      }
-    }
-    if (kTMA) {
-      if (!mbar_wait(mbar, phase)) atomicExch(s_abort, 1);
-    }
-    cp_async_wait_group<0>();
-    __syncthreads();
-    if (*s_abort) {
-      if (tid == 0) {
-        atomicAdd(&P.status->timeouts, 1ull);
-        mbar_wait(mbar, phase);  // give copies in flight one more bounded wait
-      }
-      break;
-    }
-
-    // 3. particles of this tile, CH at a time
-    constexpr int kStageFloats = (int)(G::stage_bytes() / 4);
     // 3a. coalesced asynchronous load of the chunk at c0 into buffer b
     auto issue = [&](int c0, int b) {
-      float *sb = st + b * kStageFloats;
+      float *sb = reinterpret_cast<float *>(s_stage + b * G::stage0_bytes());
       const int nch = min(CH, n_t - c0);
 #pragma unroll
       for (int k = 0; k < PER_THREAD; ++k) {
@@ -377,13 +353,65 @@ __device__ __forceinline__ void push_deposit_tiles(const PushDepositParams &P0,
       }
       cp_async_commit();
     };
+    // 1. field tile: the copies run while the current tile is zeroed and the
+    // first chunk's loads are issued
+    if (kTMA && tid == 0) {
+      fence_proxy_async_smem();
+      mbar_expect_tx(mbar, 6u * G::BX * G::BY * 4u);
+#pragma unroll
+      for (int k = 0; k < 6; ++k) tma_load_2d(sRaw + k * G::FSZ, mp + k, xs, ys, mbar);
+    }
+    // 2. zero the current (and charge) tile
+    for (int i = tid; i < nacc; i += kThreads2D) {
+      sJhi[i] = 0;
+      sJlo[i] = 0u;
+    }
+    if constexpr (kLS) {
+      for (int i = tid; i < G::JSZ; i += kThreads2D) {
+        const int gx = jx0 + i % G::JX, gy = jy0 + i / G::JX;
+        s_dv[i] = (gx < dims0 && gy < dims1) ? P.dV.ptr[(size_t)gy * P.dV.pitch + gx] : 1.0f;
+      }
+    }
+    if (G::NBUF == 2) {
+      cp_async_wait_group<0>();
+      __syncthreads();  // the order indices of the first chunks
+      if (p0 < n_t) issue(p0, 0);
+    }
+    if (kTMA) {
+      if (!mbar_wait(mbar, phase)) atomicExch(s_abort, 1);
+    }
+    for (int i = tid; i < kNodes; i += kThreads2D) {
+      const int j = i / G::RX, col = i - j * G::RX;
+      float f[6][2];
+#pragma unroll
+      for (int k = 0; k < 6; ++k)
+#pragma unroll
+        for (int d = 0; d < 2; ++d) {
+          if constexpr (kTMA) {
+            f[k][d] = sRaw[k * G::FSZ + j * G::BX + (x0 - 1 - xs) + col + d];
+          } else {
+            const int xx = x0 - 1 + col + d, yy = ys + j;
+            f[k][d] = xx < dims0 && yy < dims1 ? P.F[k].ptr[(size_t)yy * P.F[k].pitch + xx] : 0.0f;
+          }
+        }
+      sEB[i] = make_float4(f[0][0], f[0][1], f[4][0], f[4][1]);
+      sEB[kNodes + i] = make_float4(f[1][0], f[1][1], f[3][0], f[3][1]);
+      sZ[i] = make_float2(f[2][0], f[2][1]);
+      sZ[kNodes + i] = make_float2(f[5][0], f[5][1]);
+    }
+    cp_async_wait_group<0>();  // the first chunk
+    __syncthreads();
+    if (*s_abort) {
+      if (tid == 0) {
+        atomicAdd(&P.status->timeouts, 1ull);
+        mbar_wait(mbar, phase);  // give copies in flight one more bounded wait
+      }
+      break;
+    }
+
+    // 3. particles of this item, CH at a time
     int buf = 0;
     uint32_t cnt_prev = 0;  // threads < 10: the tile's direction count so far
-    if (G::NBUF == 2 && p0 < n_t) {
-      issue(p0, 0);
-      cp_async_wait_group<0>();
-      __syncthreads();
-    }
     for (int c0 = p0; c0 < n_t; c0 += CH) {
       const int nch = min(CH, n_t - c0);
       if (G::NBUF == 2) {
@@ -396,7 +424,7 @@ __device__ __forceinline__ void push_deposit_tiles(const PushDepositParams &P0,
         cp_async_wait_group<0>();
         __syncthreads();
       }
-      float *stc = st + buf * kStageFloats;
+      float *stc = reinterpret_cast<float *>(s_stage + buf * G::stage0_bytes());
       float *s_x1 = stc, *s_x2 = stc + SP, *s_x3 = stc + 2 * SP;
       float *s_p1 = stc + 3 * SP, *s_p2 = stc + 4 * SP, *s_p3 = stc + 5 * SP;
       float *s_w = stc + 6 * SP;  // weight in, gamma out
@@ -440,25 +468,34 @@ __device__ __forceinline__ void push_deposit_tiles(const PushDepositParams &P0,
             const float qm = P.qm[sp];
             const Weights1D Wx = weights_1d(x1, c1);
             const Weights1D Wy = weights_1d(x2, c2);
+            // each component: its four nodes in the reference's order, times
+            // the x weight, then the y weight, added up from zero
             float fe[6];
-#pragma unroll
-            for (int q = 0; q < 6; ++q) {
-              const float *f = sF + q * G::FSZ;
-              const int ib = (stag_x(q) ? c1 - 1 : Wx.base0) - xs;
-              const int jb = (stag_y(q) ? c2 - 1 : Wy.base0) - ys;
-              const float wx0 = stag_x(q) ? Wx.w1[0] : Wx.w0[0];
-              const float wx1 = stag_x(q) ? Wx.w1[1] : Wx.w0[1];
-              const float wy0 = stag_y(q) ? Wy.w1[0] : Wy.w0[0];
-              const float wy1 = stag_y(q) ? Wy.w1[1] : Wy.w0[1];
-              const float *row0 = f + jb * G::BX + ib;
-              const float *row1 = row0 + G::BX;
+            auto comp = [&](float2 r0, float2 r1, const float wx[2], const float wy[2]) {
+              const float2 w = make_float2(wx[0], wx[1]);
+              const float2 a = __fmul2_rn(__fmul2_rn(r0, w), make_float2(wy[0], wy[0]));
+              const float2 b = __fmul2_rn(__fmul2_rn(r1, w), make_float2(wy[1], wy[1]));
               float acc = 0.0f;
-              acc += row0[0] * wx0 * wy0;
-              acc += row0[1] * wx1 * wy0;
-              acc += row1[0] * wx0 * wy1;
-              acc += row1[1] * wx1 * wy1;
-              fe[q] = acc * qm;
+              acc += a.x;
+              acc += a.y;
+              acc += b.x;
+              acc += b.y;
+              return acc * qm;
+            };
+            const int i0 = Wx.base0 - (x0 - 1), i1 = c1 - x0;
+            const int j0 = (Wy.base0 - ys) * G::RX, j1 = (c2 - y0) * G::RX;
+            {
+              const float4 r0 = sEB[j1 + i0], r1 = sEB[j1 + G::RX + i0];
+              fe[0] = comp(make_float2(r0.x, r0.y), make_float2(r1.x, r1.y), Wx.w0, Wy.w1);
+              fe[4] = comp(make_float2(r0.z, r0.w), make_float2(r1.z, r1.w), Wx.w0, Wy.w1);
             }
+            {
+              const float4 r0 = sEB[kNodes + j0 + i1], r1 = sEB[kNodes + j0 + G::RX + i1];
+              fe[1] = comp(make_float2(r0.x, r0.y), make_float2(r1.x, r1.y), Wx.w1, Wy.w0);
+              fe[3] = comp(make_float2(r0.z, r0.w), make_float2(r1.z, r1.w), Wx.w1, Wy.w0);
+            }
+            fe[2] = comp(sZ[j1 + i1], sZ[j1 + G::RX + i1], Wx.w1, Wy.w1);
+            fe[5] = comp(sZ[kNodes + j0 + i0], sZ[kNodes + j0 + G::RX + i0], Wx.w0, Wy.w0);
             if constexpr (!kLS) {
               vay_push_v(p1, p2, p3, gamma, fe[0], fe[1], fe[2], fe[3], fe[4], fe[5], v1, v2, v3);
             } else {
@@ -782,12 +819,8 @@ __device__ __forceinline__ void push_deposit_tiles(const PushDepositParams &P0,
       atomicAdd(P.acc + comp * P.acc_comp + (size_t)gy * P.acc_pitch + gx,
                 (unsigned long long)v);
     }
-    if (tid < 10) {
-      if constexpr (kMulti)
-        P.dir_count[t * 10 + tid] = s_cnt[tid];
-      else if (s_cnt[tid])
-        atomicAdd(&P.dir_count[t * 10 + tid], s_cnt[tid]);  // a tile's items, counts start at 0
-    }
+    // the tile's other items add to the same counts, which start at 0
+    if (tid < 10 && s_cnt[tid]) atomicAdd(&P.dir_count[t * 10 + tid], s_cnt[tid]);
     phase ^= 1u;
   }
 }
@@ -1245,14 +1278,36 @@ cudaError_t launch_push_deposit_2d(Ctx &c, const PushDepositParams &P) {
 
 namespace {
 
+// First item of each run in the batch's queue, from the runs' item counts (one
+// warp); the queue starts at 0.
+__global__ void k_batch_bases(const RunDesc *__restrict__ runs, int nruns, uint32_t *base,
+                              uint32_t *queue) {
+  const int lane = threadIdx.x;
+  uint32_t carry = 0;
+  for (int r0 = 0; r0 < nruns; r0 += 32) {
+    const int r = r0 + lane;
+    const uint32_t own = r < nruns ? *runs[r].P.n_items : 0u;
+    uint32_t inc = own;
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t t = __shfl_up_sync(0xffffffffu, inc, o);
+      if (lane >= o) inc += t;
+    }
+    if (r < nruns) base[r] = carry + inc - own;
+    carry += __shfl_sync(0xffffffffu, inc, 31);
+  }
+  if (lane == 0) {
+    base[nruns] = carry;
+    *queue = 0u;
+  }
+}
+
 template <int TX, int TY, int CH, int MINB>
 cudaError_t launch_batch_tiles(cudaStream_t stream, int num_sms, bool tma, bool do_rho,
-                               int max_species, const RunDesc *runs, const uint32_t *base,
+                               int max_species, const RunDesc *runs, uint32_t *base,
                                int nruns, uint32_t total, uint32_t *queue) {
   using G = TileGeom<TX, TY, CH>;
   const size_t smem = G::smem_bytes(do_rho ? max_species : 0);
-  cudaError_t e = cudaMemsetAsync(queue, 0, sizeof(uint32_t), stream);
-  if (e != cudaSuccess) return e;
+  k_batch_bases<<<1, 32, 0, stream>>>(runs, nruns, base, queue);
   auto run = [&](auto kern) -> cudaError_t {
     cudaError_t err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                            (int)smem);
@@ -1277,7 +1332,7 @@ cudaError_t launch_batch_tiles(cudaStream_t stream, int num_sms, bool tma, bool 
 template <int TX, int TY>
 cudaError_t launch_batch_chunk(cudaStream_t stream, int num_sms, int chunk, bool tma,
                                bool do_rho, int max_species, const RunDesc *runs,
-                               const uint32_t *base, int nruns, uint32_t total,
+                               uint32_t *base, int nruns, uint32_t total,
                                uint32_t *queue) {
   if (chunk == 2048)
     return launch_batch_tiles<TX, TY, 2048, 2>(stream, num_sms, tma, do_rho, max_species, runs,
@@ -1296,7 +1351,7 @@ cudaError_t launch_batch_chunk(cudaStream_t stream, int num_sms, int chunk, bool
 
 cudaError_t launch_push_deposit_2d_batch(cudaStream_t stream, int num_sms, int tx, int ty,
                                          int chunk, bool tma, bool do_rho, int max_species,
-                                         const RunDesc *runs, const uint32_t *base, int nruns,
+                                         const RunDesc *runs, uint32_t *base, int nruns,
                                          uint32_t total, uint32_t *queue) {
   if (total == 0) return cudaSuccess;
 #define AP_BATCH_SHAPE(X, Y)                                                                 \

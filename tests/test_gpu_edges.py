@@ -1,0 +1,121 @@
+"""GPU parity at the edges of the update's fast paths: the shared-reciprocal
+quotients of the Vay push at the limits of their range, work items of tile
+lists (crowded, single and empty tiles, lists around a chunk's length), the 1D
+kernel's chunk lengths, the one-launch field update at its size limit and the
+smoothing passes of mixed boundaries. Particles, fields and smoothed currents
+bit for bit against the oracle, J and Rho within 1e-6 of their maximum of the
+FP64-accumulated deposit (one FP32 rounding of an exact sum of FP32
+contributions, 6e-8 each)."""
+import numpy as np
+import pytest
+
+import oracle
+from _cases import random_fields, random_particles
+from _gpu_helpers import Pair, assert_bits, make_params
+
+pytestmark = pytest.mark.gpu
+
+J_TOL = 1e-6
+
+
+def _state(N, n, seed, amp=0.3, periodic=(True, True), smoothing=0, tile=(0, 0)):
+    params = make_params(N, periodic=periodic, capacity=max(n, 1), tile=tile,
+                         smoothing=smoothing)
+    m = oracle.make_mesh(params.N, params.guard, size=params.size)
+    rng = np.random.default_rng(seed)
+    f = random_fields(m, rng, amp=amp)
+    for key in ("E", "B", "Ebg", "Bbg"):
+        for c in range(3):
+            oracle.send_guard_cells(m, f[key][c], (1, 1, 0))
+    return params, m, rng, f
+
+
+@pytest.mark.parametrize("N", [(64, 48), (512,)])
+@pytest.mark.parametrize("amp", [0.0, 1e-34, 0.3, 3e4, 1e7])
+def test_push_quotients_at_their_range(N, amp):
+    """Zero, denormal, tiny, large and huge momentum components (gamma past
+    2^24 too) in zero, tiny, ordinary and huge fields: the quotients by gamma
+    equal the plain divisions on both sides of every bound."""
+    params, m, rng, f = _state(N, 6000, 3, amp=amp)
+    p = random_particles(m, 6000, rng)
+    sizes = np.array([0.0, 1e-42, 3e-39, 7e-31, 8e-31, 1e-20, 1.0, 1e3, 1.6e7, 1.7e7, 1e9],
+                     np.float32)
+    for k in ("p1", "p2", "p3"):
+        sgn = np.where(rng.random(6000) < 0.5, -1, 1).astype(np.float32)
+        p[k][:] = sgn * sizes[rng.integers(0, len(sizes), 6000)] * (
+            1 + rng.random(6000, dtype=np.float32))
+    pr = Pair(params, f, p)
+    pr.both_update_particles(0)
+    pr.check_particles()
+
+
+@pytest.mark.parametrize("tile", [(16, 16), (4, 4)])
+@pytest.mark.parametrize("n", [1, 255, 256, 257, 40000])
+@pytest.mark.parametrize("crowd", [False, True])
+def test_2d_work_items(tile, n, crowd):
+    """Tile lists cut into work items of whole chunks: all particles in one
+    tile (the others empty), or spread; lists of a chunk's length and one
+    around it. Three steps keep the tile order that the items index."""
+    params, m, rng, f = _state((64, 48), n, 11, tile=tile)
+    p = random_particles(m, n, rng, gamma_max=5.0)
+    if crowd:
+        c1 = rng.integers(18, 20, n)
+        c2 = rng.integers(18, 20, n)
+        p["cell"][:] = (c1 + c2 * m.dims[0]).astype(np.uint32)
+    pr = Pair(params, f, p)
+    for step in range(3):
+        pr.both_update_particles(step)
+        pr.check_particles()
+        pr.check_current(J_TOL, rho=True)
+
+
+@pytest.mark.parametrize("n", [1, 257, 20000, 148 * 1024, 148 * 1024 * 2 + 3])
+def test_1d_chunk_lengths(n):
+    params, m, rng, f = _state((512,), n, 5)
+    p = random_particles(m, n, rng, gamma_max=5.0)
+    pr = Pair(params, f, p)
+    pr.both_update_particles(0)
+    pr.check_particles()
+    pr.check_current(J_TOL, rho=True)
+
+
+@pytest.mark.parametrize("N", [(64, 64), (64, 65), (4096,), (4097,), (5, 7)])
+def test_update_fields_at_the_small_grid_limit(N):
+    params, m, rng, f = _state(N, 1, 4)
+    for c in range(3):
+        f["J"][c][:] = (0.1 * rng.standard_normal(f["J"][c].shape)).astype(np.float32)
+    pr = Pair(params, f, random_particles(m, 0, rng))
+    g0, g1 = m.guard[0], m.guard[1]
+    sl = ((slice(g1, m.dims[1] - g1) if m.dimension > 1 else slice(0, 1)),
+          slice(g0, m.dims[0] - g0))
+    for step in range(2):
+        pr.both_update_fields(step)
+        g = pr.data.fields_host()
+        for key in ("E", "B"):
+            for c in range(3):
+                assert_bits(g[key][c], pr.f[key][c], f"{key}{c + 1} step {step}")
+        for key in ("divE", "divB"):
+            assert_bits(g[key][sl], pr.f[key][sl], key)
+
+
+@pytest.mark.parametrize("N,periodic", [((33, 21), (True, True)), ((33, 21), (True, False)),
+                                        ((33, 21), (False, True)), ((33, 21), (False, False)),
+                                        ((300,), (True, True)), ((300,), (False, True))])
+def test_smooth_current_bitexact(N, periodic):
+    """J and Rho given as arrays: two smoothing passes with the guards of the
+    periodic dims refreshed after each, in dim order, guard rows of the other
+    dim included."""
+    params, m, rng, f = _state(N, 1, 9, periodic=periodic, smoothing=2)
+    pr = Pair(params, f, random_particles(m, 0, rng))
+    per = pr.periodic
+    bnd = [int(not per[0]), int(not per[0]), int(not per[1]), int(not per[1])]
+    arrs = [rng.standard_normal(pr.f["J"][0].shape).astype(np.float32) for _ in range(5)]
+    pr.data.set_fields({"J": arrs[:3], "Rho": arrs[3:]})
+    pr.pusher.smooth_current(pr.data, 0)
+    g = pr.data.fields_host()
+    for k, a in enumerate(arrs):
+        ref = a.copy()
+        for _ in range(2):
+            oracle.filter_current(m, ref, ref.copy(), bnd)
+            oracle.send_guard_cells(m, ref, per)
+        assert_bits((g["J"] + g["Rho"])[k], ref, f"array {k}")
