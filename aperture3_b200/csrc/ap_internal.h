@@ -345,6 +345,11 @@ cudaError_t rebuild_tile_order(Ctx &c);
 // bits of the keys, ping-ponging with keys[1] / vals[1] (k_radix.cu).
 cudaError_t radix_sort_pairs(Ctx &c, size_t n, int end_bit, uint32_t **keys_out,
                              uint32_t **vals_out);
+// Stable sort of slots base + [0, n) by cell: keys = cells, `empty` for empty
+// slots and slots at or past *d_number (when given), values = slots.
+cudaError_t radix_sort_cells(Ctx &c, const uint32_t *cell, size_t base, size_t n, uint32_t empty,
+                             const uint32_t *d_number, int end_bit, uint32_t **keys_out,
+                             uint32_t **vals_out);
 size_t radix_count_words(int num_sms);
 cudaError_t sort_by_cell(Ctx &c, size_t *new_number);
 cudaError_t sort_photons(Ctx &c, size_t *new_number);

@@ -22,6 +22,8 @@
 // (cuda/core/particle_base_impl.cu:435-487) use a stable LSD radix sort.
 #include <cuda_runtime.h>
 
+#include <type_traits>
+
 #include "ap_device.cuh"
 #include "ap_internal.h"
 
@@ -484,24 +486,70 @@ __global__ void __launch_bounds__(kScanThreads)
 }
 static_assert(kScanThreads == 1024, "one warp scans the 32 warp sums");
 
-// Keys of slots base + i, i < n (vals = the slots); slots at or beyond a
-// device-side live count are empty.
-__global__ void k_cell_keys(const uint32_t *cell, size_t base, size_t n, uint32_t ncells,
-                            uint32_t *keys, uint32_t *vals, const uint32_t *d_number) {
-  const size_t live = d_number ? (size_t)*d_number : base + n;
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n;
-       i += (size_t)gridDim.x * blockDim.x) {
-    const uint32_t c = base + i < live ? cell[base + i] : AP_MAX_CELL;
-    keys[i] = (c == AP_MAX_CELL) ? ncells : c;
-    vals[i] = (uint32_t)(base + i);
-  }
-}
-
+// dst[i] = src[perm[i]], one entry per thread and round: for members larger
+// than the L2, whose sources must stay close together in it.
 template <typename T>
-__global__ void k_gather(const T *src, const uint32_t *perm, size_t n, T *dst) {
+__global__ void k_gather(const T *__restrict__ src, const uint32_t *__restrict__ perm, size_t n,
+                         T *__restrict__ dst) {
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n;
        i += (size_t)gridDim.x * blockDim.x)
     dst[i] = src[perm[i]];
+}
+
+// The same with four consecutive entries per thread: the permutation and the
+// result move 16 bytes at a time and four gathers are in flight. The first
+// `head` entries, up to dst's 16-byte boundary, go one by one; with a head the
+// permutation's words are read singly.
+template <typename T>
+__global__ void k_gather4(const T *__restrict__ src, const uint32_t *__restrict__ perm, size_t n,
+                          T *__restrict__ dst, int head) {
+  const size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
+  const size_t stride = (size_t)gridDim.x * blockDim.x * 4;
+  if (t < (size_t)head && t < n) dst[t] = src[perm[t]];
+  for (size_t i = head + t * 4; i < n; i += stride) {
+    if (i + 3 < n) {
+      uint4 q;
+      if (head == 0)
+        q = *reinterpret_cast<const uint4 *>(perm + i);
+      else
+        q = make_uint4(perm[i], perm[i + 1], perm[i + 2], perm[i + 3]);
+      const T a = src[q.x], b = src[q.y], c = src[q.z], d = src[q.w];
+      if constexpr (sizeof(T) == 4) {
+        *reinterpret_cast<uint4 *>(dst + i) = make_uint4(a, b, c, d);
+      } else {
+        *reinterpret_cast<ulonglong2 *>(dst + i) = make_ulonglong2(a, b);
+        *reinterpret_cast<ulonglong2 *>(dst + i + 2) = make_ulonglong2(c, d);
+      }
+    } else {
+      for (size_t j = i; j < n; ++j) dst[j] = src[perm[j]];
+    }
+  }
+}
+
+// The cells of a sorted store from the sort's keys (16 bytes at a time where
+// the cell array allows it).
+__global__ void k_cells_of_keys(const uint32_t *__restrict__ keys, size_t n, uint32_t empty,
+                                uint32_t *__restrict__ cell, bool vec) {
+  const size_t stride = (size_t)gridDim.x * blockDim.x * 4;
+  for (size_t i = (blockIdx.x * (size_t)blockDim.x + threadIdx.x) * 4; i < n; i += stride) {
+    if (i + 3 < n) {
+      uint4 q = *reinterpret_cast<const uint4 *>(keys + i);
+      q.x = q.x == empty ? AP_MAX_CELL : q.x;
+      q.y = q.y == empty ? AP_MAX_CELL : q.y;
+      q.z = q.z == empty ? AP_MAX_CELL : q.z;
+      q.w = q.w == empty ? AP_MAX_CELL : q.w;
+      if (vec) {
+        *reinterpret_cast<uint4 *>(cell + i) = q;
+      } else {
+        cell[i] = q.x;
+        cell[i + 1] = q.y;
+        cell[i + 2] = q.z;
+        cell[i + 3] = q.w;
+      }
+    } else {
+      for (size_t j = i; j < n; ++j) cell[j] = keys[j] == empty ? AP_MAX_CELL : keys[j];
+    }
+  }
 }
 
 int bits_for(uint32_t maxkey) {
@@ -516,6 +564,37 @@ int grid_for(Ctx &c, size_t n, int threads) {
   if (g > cap) g = cap;
   if (g < 1) g = 1;
   return (int)g;
+}
+
+// One member gathered by the sort's permutation (4- and 8-byte members move as
+// bits).
+cudaError_t gather_member(Ctx &c, const void *src, const uint32_t *perm, size_t n, int bytes,
+                          void *dst) {
+  const int off = (int)(reinterpret_cast<uintptr_t>(dst) & 15u);
+  const int head = off ? (16 - off) / bytes : 0;  // an 8-byte member starts at 0 or 8
+  // four entries per thread while the member fits the 126 MB L2: 8.4 M 4-byte
+  // members 32 -> 19 us, 16.8 M 62 -> 55 us; past it their sources, in a store
+  // in tile order, spread too far: 67 M 264 -> 286 us, 8-byte 339 -> 635 us
+  const bool four = n * (size_t)bytes <= (size_t)128 << 20;
+  auto run = [&](auto *s, auto *d) {
+    using T = std::remove_pointer_t<decltype(d)>;
+    if (four)
+      k_gather4<T><<<grid_for(c, (n + 3) / 4, 256), 256, 0, c.stream>>>(s, perm, n, d, head);
+    else
+      k_gather<T><<<grid_for(c, n, 256), 256, 0, c.stream>>>(s, perm, n, d);
+  };
+  if (bytes == 8)
+    run(static_cast<const uint64_t *>(src), static_cast<uint64_t *>(dst));
+  else
+    run(static_cast<const uint32_t *>(src), static_cast<uint32_t *>(dst));
+  c.launches++;
+  return cudaGetLastError();
+}
+
+void launch_cells_of_keys(Ctx &c, const uint32_t *keys, size_t n, uint32_t empty, uint32_t *cell) {
+  const bool vec = (reinterpret_cast<uintptr_t>(cell) & 15u) == 0;
+  k_cells_of_keys<<<grid_for(c, (n + 3) / 4, 256), 256, 0, c.stream>>>(keys, n, empty, cell, vec);
+  c.launches++;
 }
 
 // Stable radix sort of (keys[0], vals[0]) -> result pointers (k_radix.cu).
@@ -614,7 +693,7 @@ __global__ void k_compact_tail(const uint32_t *live, uint32_t *cell, size_t n) {
   const uint32_t m = *live;
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n;
        i += (size_t)gridDim.x * blockDim.x)
-    if (i >= m) cell[i] = AP_MAX_CELL;
+    cell[i] = AP_MAX_CELL;
 }
 
 namespace {
@@ -788,15 +867,11 @@ cudaError_t sort_by_cell(Ctx &c, size_t *new_number) {
   }
   const uint32_t ncells =
       (uint32_t)c.mesh.dims[0] * (uint32_t)c.mesh.dims[1] * (uint32_t)c.mesh.dims[2];
-  k_cell_keys<<<grid_for(c, n, 256), 256, 0, c.stream>>>(c.ptc.cell, base, n, ncells, c.keys[0],
-                                                        c.vals[0],
-                                                        device_count ? &c.pstate->number
-                                                                     : nullptr);
-  c.launches++;
   uint32_t *ko, *vo;
-  cudaError_t e = radix_pairs(c, n, bits_for(ncells), &ko, &vo);
+  cudaError_t e = radix_sort_cells(c, c.ptc.cell, base, n, ncells,
+                                   device_count ? &c.pstate->number : nullptr, bits_for(ncells),
+                                   &ko, &vo);
   if (e != cudaSuccess) return e;
-  const int g = grid_for(c, n, 256);
   // With compaction on and a free half of the capacity, each member is
   // gathered straight into that half (the store then occupies
   // [out0, out0 + live)); otherwise through the gather buffer and back to
@@ -815,30 +890,24 @@ cudaError_t sort_by_cell(Ctx &c, size_t *new_number) {
       out0 = 0;
     }
   }
-#define AP_GATHER(FIELD, T)                                                                  \
-  do {                                                                                        \
-    if (direct) {                                                                             \
-      k_gather<T><<<g, 256, 0, c.stream>>>(c.ptc.FIELD, vo, n, (T *)c.ptc.FIELD + out0);      \
-    } else {                                                                                  \
-      k_gather<T><<<g, 256, 0, c.stream>>>(c.ptc.FIELD, vo, n, (T *)c.gather_tmp);           \
-      e = cudaMemcpyAsync(c.ptc.FIELD, c.gather_tmp, n * sizeof(T), cudaMemcpyDeviceToDevice, \
-                          c.stream);                                                          \
-      if (e != cudaSuccess) return e;                                                         \
-    }                                                                                         \
-    c.launches++;                                                                             \
-  } while (0)
-  AP_GATHER(x1, float);
-  AP_GATHER(x2, float);
-  AP_GATHER(x3, float);
-  AP_GATHER(p1, float);
-  AP_GATHER(p2, float);
-  AP_GATHER(p3, float);
-  AP_GATHER(E, float);
-  AP_GATHER(weight, float);
-  AP_GATHER(cell, uint32_t);
-  AP_GATHER(id, uint64_t);
-  AP_GATHER(flag, uint32_t);
-#undef AP_GATHER
+  const struct {
+    void *p;
+    int bytes;
+  } member[10] = {{c.ptc.x1, 4}, {c.ptc.x2, 4}, {c.ptc.x3, 4},     {c.ptc.p1, 4}, {c.ptc.p2, 4},
+                  {c.ptc.p3, 4}, {c.ptc.E, 4},  {c.ptc.weight, 4}, {c.ptc.id, 8}, {c.ptc.flag, 4}};
+  for (const auto &m : member) {
+    unsigned char *p = static_cast<unsigned char *>(m.p);
+    if (direct) {
+      e = gather_member(c, p, vo, n, m.bytes, p + out0 * m.bytes);
+    } else {
+      e = gather_member(c, p, vo, n, m.bytes, c.gather_tmp);
+      if (e == cudaSuccess)
+        e = cudaMemcpyAsync(p, c.gather_tmp, n * m.bytes, cudaMemcpyDeviceToDevice, c.stream);
+    }
+    if (e != cudaSuccess) return e;
+  }
+  // the cells are the sort's keys: no gather, and no copy back
+  launch_cells_of_keys(c, ko, n, ncells, c.ptc.cell + (direct ? out0 : 0));
   if (direct && out0 > 0) {  // the old particles sat below the new range: empty them
     e = cudaMemsetAsync(c.ptc.cell, 0xff, c.number * sizeof(uint32_t), c.stream);
     if (e != cudaSuccess) return e;
@@ -883,34 +952,22 @@ cudaError_t sort_photons(Ctx &c, size_t *new_number) {
   if (ensure_scratch(c, n) != AP_OK) return cudaErrorMemoryAllocation;
   const uint32_t ncells =
       (uint32_t)c.mesh.dims[0] * (uint32_t)c.mesh.dims[1] * (uint32_t)c.mesh.dims[2];
-  k_cell_keys<<<grid_for(c, n, 256), 256, 0, c.stream>>>(c.ph.cell, 0, n, ncells, c.keys[0],
-                                                        c.vals[0], nullptr);
-  c.launches++;
   uint32_t *ko, *vo;
-  cudaError_t e = radix_pairs(c, n, bits_for(ncells), &ko, &vo);
+  cudaError_t e = radix_sort_cells(c, c.ph.cell, 0, n, ncells, nullptr, bits_for(ncells), &ko, &vo);
   if (e != cudaSuccess) return e;
-  const int g = grid_for(c, n, 256);
-#define AP_GATHER_PH(FIELD, T)                                                                \
-  do {                                                                                        \
-    k_gather<T><<<g, 256, 0, c.stream>>>(c.ph.FIELD, vo, n, (T *)c.gather_tmp);               \
-    e = cudaMemcpyAsync(c.ph.FIELD, c.gather_tmp, n * sizeof(T), cudaMemcpyDeviceToDevice,    \
-                        c.stream);                                                            \
-    if (e != cudaSuccess) return e;                                                           \
-    c.launches++;                                                                             \
-  } while (0)
-  AP_GATHER_PH(x1, float);
-  AP_GATHER_PH(x2, float);
-  AP_GATHER_PH(x3, float);
-  AP_GATHER_PH(p1, float);
-  AP_GATHER_PH(p2, float);
-  AP_GATHER_PH(p3, float);
-  AP_GATHER_PH(E, float);
-  AP_GATHER_PH(weight, float);
-  AP_GATHER_PH(path_left, float);
-  AP_GATHER_PH(cell, uint32_t);
-  AP_GATHER_PH(id, uint64_t);
-  AP_GATHER_PH(flag, uint32_t);
-#undef AP_GATHER_PH
+  const struct {
+    void *p;
+    int bytes;
+  } member[11] = {{c.ph.x1, 4}, {c.ph.x2, 4}, {c.ph.x3, 4},     {c.ph.p1, 4},
+                  {c.ph.p2, 4}, {c.ph.p3, 4}, {c.ph.E, 4},      {c.ph.weight, 4},
+                  {c.ph.path_left, 4},        {c.ph.id, 8},     {c.ph.flag, 4}};
+  for (const auto &m : member) {
+    e = gather_member(c, m.p, vo, n, m.bytes, c.gather_tmp);
+    if (e == cudaSuccess)
+      e = cudaMemcpyAsync(m.p, c.gather_tmp, n * m.bytes, cudaMemcpyDeviceToDevice, c.stream);
+    if (e != cudaSuccess) return e;
+  }
+  launch_cells_of_keys(c, ko, n, ncells, c.ph.cell);
   if (!c.cell_start) {
     e = cudaMalloc(&c.cell_start, sizeof(uint32_t) * ((size_t)ncells + 1));
     if (e != cudaSuccess) return e;

@@ -119,3 +119,30 @@ def test_smooth_current_bitexact(N, periodic):
             oracle.filter_current(m, ref, ref.copy(), bnd)
             oracle.send_guard_cells(m, ref, per)
         assert_bits((g["J"] + g["Rho"])[k], ref, f"array {k}")
+
+
+@pytest.mark.parametrize("n,order", [(1, "random"), (3, "random"), (4095, "random"),
+                                     (4097, "cells"), (70001, "random"), (70002, "cells"),
+                                     (70003, "reverse")])
+@pytest.mark.parametrize("half", [False, True])
+def test_sort_by_cell_around_its_tiles(n, order, half):
+    """sort_by_cell of random, cell-ordered and reversed stores with empty
+    slots, in place and into the other half of the capacity (whose start is
+    not 16-byte aligned for odd n): every member equals the stable sort."""
+    params, m, rng, _ = _state((40, 24), n, 21)
+    p = random_particles(m, n, rng)
+    if order != "random":
+        perm = np.argsort(p["cell"], kind="stable")
+        for k in p:
+            p[k][:] = p[k][perm if order == "cells" else perm[::-1]]
+    p["cell"][rng.random(n) < 0.05] = oracle.MAX_CELL
+    pr = Pair(params, {}, p, capacity=2 * n if half else n)
+    if half:
+        pr.env.set_compaction(2)
+    pr.data.sort_particles()
+    n_ref = oracle.sort_by_cell(m, pr.p, n)
+    first, end = pr.data.slot_range()
+    assert (first, end) == ((n, n + n_ref) if half else (0, n_ref))
+    got = {k: v[first:end] for k, v in pr.data.particles_host().items()}
+    for k, _ in oracle.PTC_FIELDS:
+        assert_bits(got[k], pr.p[k][:n_ref], f"sorted {k}")
