@@ -507,10 +507,15 @@ int update_particles_gap(Ctx *c, double dt, uint32_t step) {
   AP_TRY(cudaMemsetAsync(c->status, 0, sizeof(DevStatus), c->stream));
   // E3 = E1, smoothed current_smoothing times through E2 (:232-240)
   float *E1 = c->fields.E[0].ptr, *E2 = c->fields.E[1].ptr, *E3 = c->fields.E[2].ptr;
-  AP_TRY(cudaMemcpyAsync(E3, E1, sizeof(float) * n, cudaMemcpyDeviceToDevice, c->stream));
-  for (int it = 0; it < pr.current_smoothing; ++it) {
-    AP_TRY(launch_gap_filter(*c, E3, E2, bl, bu));
-    AP_TRY(cudaMemcpyAsync(E3, E2, sizeof(float) * n, cudaMemcpyDeviceToDevice, c->stream));
+  const bool fits = line_smooth_fits(*c);
+  if (fits) {
+    AP_TRY(launch_line_smooth_e(*c, nullptr, pr.current_smoothing));
+  } else {
+    AP_TRY(cudaMemcpyAsync(E3, E1, sizeof(float) * n, cudaMemcpyDeviceToDevice, c->stream));
+    for (int it = 0; it < pr.current_smoothing; ++it) {
+      AP_TRY(launch_gap_filter(*c, E3, E2, bl, bu));
+      AP_TRY(cudaMemcpyAsync(E3, E2, sizeof(float) * n, cudaMemcpyDeviceToDevice, c->stream));
+    }
   }
   phase_end(c, ph);
   PushDepositParams P;
@@ -544,15 +549,19 @@ int update_particles_gap(Ctx *c, double dt, uint32_t step) {
   ph = phase_begin(c, kPhFinalize);
   AP_TRY(launch_finalize_current(*c, ncomp));
   // J1 and each Rho smoothed current_smoothing times (:254-268)
-  float *tmp = c->tmp_j;
-  for (int it = 0; it < pr.current_smoothing; ++it) {
-    AP_TRY(launch_gap_filter(*c, c->fields.J[0].ptr, tmp, bl, bu));
-    AP_TRY(cudaMemcpyAsync(c->fields.J[0].ptr, tmp, sizeof(float) * n, cudaMemcpyDeviceToDevice,
-                           c->stream));
-    for (int s = 0; s < pr.num_species; ++s) {
-      AP_TRY(launch_gap_filter(*c, c->fields.Rho[s].ptr, tmp, bl, bu));
-      AP_TRY(cudaMemcpyAsync(c->fields.Rho[s].ptr, tmp, sizeof(float) * n,
-                             cudaMemcpyDeviceToDevice, c->stream));
+  if (fits) {
+    AP_TRY(launch_line_smooth_current(*c, nullptr, nullptr, pr.current_smoothing));
+  } else {
+    float *tmp = c->tmp_j;
+    for (int it = 0; it < pr.current_smoothing; ++it) {
+      AP_TRY(launch_gap_filter(*c, c->fields.J[0].ptr, tmp, bl, bu));
+      AP_TRY(cudaMemcpyAsync(c->fields.J[0].ptr, tmp, sizeof(float) * n, cudaMemcpyDeviceToDevice,
+                             c->stream));
+      for (int s = 0; s < pr.num_species; ++s) {
+        AP_TRY(launch_gap_filter(*c, c->fields.Rho[s].ptr, tmp, bl, bu));
+        AP_TRY(cudaMemcpyAsync(c->fields.Rho[s].ptr, tmp, sizeof(float) * n,
+                               cudaMemcpyDeviceToDevice, c->stream));
+      }
     }
   }
   c->rho_is_zero = false;
@@ -582,10 +591,15 @@ int update_particles_gr(Ctx *c, double dt, uint32_t step) {
   AP_TRY(cudaMemsetAsync(c->status, 0, sizeof(DevStatus), c->stream));
   // E3 = E1, smoothed current_smoothing times through E2 with K1_j (:428-435)
   float *E1 = c->fields.E[0].ptr, *E2 = c->fields.E[1].ptr, *E3 = c->fields.E[2].ptr;
-  AP_TRY(cudaMemcpyAsync(E3, E1, sizeof(float) * n, cudaMemcpyDeviceToDevice, c->stream));
-  for (int it = 0; it < pr.current_smoothing; ++it) {
-    AP_TRY(launch_gr_filter(*c, E3, E2, K1j, bl, bu));
-    AP_TRY(cudaMemcpyAsync(E3, E2, sizeof(float) * n, cudaMemcpyDeviceToDevice, c->stream));
+  const bool fits = line_smooth_fits(*c);
+  if (fits) {
+    AP_TRY(launch_line_smooth_e(*c, K1j, pr.current_smoothing));
+  } else {
+    AP_TRY(cudaMemcpyAsync(E3, E1, sizeof(float) * n, cudaMemcpyDeviceToDevice, c->stream));
+    for (int it = 0; it < pr.current_smoothing; ++it) {
+      AP_TRY(launch_gr_filter(*c, E3, E2, K1j, bl, bu));
+      AP_TRY(cudaMemcpyAsync(E3, E2, sizeof(float) * n, cudaMemcpyDeviceToDevice, c->stream));
+    }
   }
   phase_end(c, ph);
   PushDepositParams P;
@@ -633,15 +647,19 @@ int update_particles_gr(Ctx *c, double dt, uint32_t step) {
   ph = phase_begin(c, kPhFinalize);
   AP_TRY(launch_finalize_current(*c, ncomp));
   // J1 (K1_j) and each Rho (K1) smoothed current_smoothing times (:447-466)
-  float *tmp = c->tmp_j;
-  for (int it = 0; it < pr.current_smoothing; ++it) {
-    AP_TRY(launch_gr_filter(*c, c->fields.J[0].ptr, tmp, K1j, bl, bu));
-    AP_TRY(cudaMemcpyAsync(c->fields.J[0].ptr, tmp, sizeof(float) * n, cudaMemcpyDeviceToDevice,
-                           c->stream));
-    for (int s = 0; s < pr.num_species; ++s) {
-      AP_TRY(launch_gr_filter(*c, c->fields.Rho[s].ptr, tmp, K1, bl, bu));
-      AP_TRY(cudaMemcpyAsync(c->fields.Rho[s].ptr, tmp, sizeof(float) * n,
-                             cudaMemcpyDeviceToDevice, c->stream));
+  if (fits) {
+    AP_TRY(launch_line_smooth_current(*c, K1j, K1, pr.current_smoothing));
+  } else {
+    float *tmp = c->tmp_j;
+    for (int it = 0; it < pr.current_smoothing; ++it) {
+      AP_TRY(launch_gr_filter(*c, c->fields.J[0].ptr, tmp, K1j, bl, bu));
+      AP_TRY(cudaMemcpyAsync(c->fields.J[0].ptr, tmp, sizeof(float) * n, cudaMemcpyDeviceToDevice,
+                             c->stream));
+      for (int s = 0; s < pr.num_species; ++s) {
+        AP_TRY(launch_gr_filter(*c, c->fields.Rho[s].ptr, tmp, K1, bl, bu));
+        AP_TRY(cudaMemcpyAsync(c->fields.Rho[s].ptr, tmp, sizeof(float) * n,
+                               cudaMemcpyDeviceToDevice, c->stream));
+      }
     }
   }
   c->rho_is_zero = false;

@@ -367,6 +367,10 @@ cudaError_t launch_divs(Ctx &c);
 cudaError_t launch_fields(Ctx &c, float dt, float dt_half);
 cudaError_t launch_filter(Ctx &c, ap_array a, int bnd[4]);
 cudaError_t launch_smooth_current(Ctx &c, bool with_rho, const int bnd[4]);
+// 1D labs: smoothing of whole rows in one launch, for rows that fit
+bool line_smooth_fits(const Ctx &c);
+cudaError_t launch_line_smooth_e(Ctx &c, const float *k1, int passes);
+cudaError_t launch_line_smooth_current(Ctx &c, const float *kj, const float *kr, int passes);
 cudaError_t launch_zero(Ctx &c, ap_array a);
 cudaError_t launch_finalize_current(Ctx &c, int ncomp);
 cudaError_t launch_fixed_scale(Ctx &c);

@@ -611,6 +611,97 @@ cudaError_t launch_smooth_current(Ctx &c, bool with_rho, const int bnd[4]) {
   return smooth_pass(c, A, n, reinterpret_cast<float *>(c.acc), 2 * c.acc_comp, bnd, true);
 }
 
+// ---------------------------------------------------------------------------
+// The 1D labs' smoothing (gap: 1-2-1 over whole rows, ptc_updater_1dgap.cu:
+// 196-213; GR: weighted by a flux-tube factor and divided by the cell's own,
+// ptc_updater_1dgr.cu:388-404): all passes of several rows in one launch, one
+// CTA per row, the row in shared memory between the passes (two buffers). The
+// value past either end of a row counts as 0.
+struct LineRow {
+  const float *src;
+  float *dst, *dst2;    // dst2: a second copy of the result, or null
+  const float *k1;      // GR: the weights; null: the gap lab's filter
+};
+struct LineRows {
+  LineRow r[2 + AP_MAX_SPECIES];
+};
+constexpr int kLineThreads = 512;
+
+__global__ void __launch_bounds__(kLineThreads)
+    k_line_smooth(const __grid_constant__ LineRows R, int n, int g, int bnd_lower, int bnd_upper,
+                  int passes) {
+  extern __shared__ float s_line[];
+  const LineRow &row = R.r[blockIdx.x];
+  float *a = s_line, *b = s_line + n;
+  for (int i = threadIdx.x; i < n; i += kLineThreads) a[i] = row.src[i];
+  __syncthreads();
+  for (int it = 0; it < passes; ++it) {
+    for (int i = threadIdx.x; i < n; i += kLineThreads) {
+      const int ip = i + ((bnd_upper && i == n - g - 1) ? 0 : 1);
+      const int im = i - ((bnd_lower && i == g) ? 0 : 1);
+      const float jp = ip < n ? a[ip] : 0.0f, jm = im >= 0 ? a[im] : 0.0f;
+      float t;
+      if (row.k1) {
+        const float kp = ip < n ? row.k1[ip] : 0.0f, km = im >= 0 ? row.k1[im] : 0.0f;
+        t = 0.5f * a[i] * row.k1[i];
+        t += 0.25f * jp * kp;
+        t += 0.25f * jm * km;
+        t /= row.k1[i];
+      } else {
+        t = 0.5f * a[i];
+        t += 0.25f * jp;
+        t += 0.25f * jm;
+      }
+      b[i] = t;
+    }
+    __syncthreads();
+    float *t = a;
+    a = b;
+    b = t;
+  }
+  for (int i = threadIdx.x; i < n; i += kLineThreads) {
+    row.dst[i] = a[i];
+    if (row.dst2) row.dst2[i] = a[i];
+  }
+}
+
+// Rows that fit shared memory twice: up to 28000 cells in one launch for all
+// rows and passes. 8192 cells, one pass of E3, J1 and two charge densities:
+// 9 launches of 1.6 us before, 2 here.
+bool line_smooth_fits(const Ctx &c) { return c.mesh.dims[0] <= 28000; }
+
+static cudaError_t launch_line_rows(Ctx &c, const LineRows &R, int rows, int passes) {
+  const size_t smem = 2 * sizeof(float) * (size_t)c.mesh.dims[0];
+  if (smem > 48 * 1024) {
+    cudaError_t e = cudaFuncSetAttribute(k_line_smooth,
+                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+  }
+  const int b = !c.params.periodic[0];
+  k_line_smooth<<<rows, kLineThreads, smem, c.stream>>>(R, c.mesh.dims[0], c.mesh.guard[0], b, b,
+                                                        passes);
+  c.launches++;
+  return cudaGetLastError();
+}
+
+// E3 = E1 smoothed `passes` times, the scratch E2 a copy of it when passes > 0.
+cudaError_t launch_line_smooth_e(Ctx &c, const float *k1, int passes) {
+  LineRows R{};
+  R.r[0] = LineRow{c.fields.E[0].ptr, c.fields.E[2].ptr,
+                   passes > 0 ? c.fields.E[1].ptr : nullptr, k1};
+  return launch_line_rows(c, R, 1, passes);
+}
+
+// J1 (weights kj) and every charge density (weights kr) smoothed in place.
+cudaError_t launch_line_smooth_current(Ctx &c, const float *kj, const float *kr, int passes) {
+  if (passes <= 0) return cudaSuccess;
+  LineRows R{};
+  R.r[0] = LineRow{c.fields.J[0].ptr, c.fields.J[0].ptr, nullptr, kj};
+  for (int s = 0; s < c.params.num_species; ++s)
+    R.r[1 + s] = LineRow{c.fields.Rho[s].ptr, c.fields.Rho[s].ptr, nullptr, kr};
+  return launch_line_rows(c, R, 1 + c.params.num_species, passes);
+}
+
 cudaError_t launch_finalize_current(Ctx &c, int ncomp) {
   Geo G = make_geo(c);
   Arr o[11];

@@ -91,16 +91,36 @@ __device__ void gap_chunk(const PushDepositParams &P, size_t ch, int *sWhi, unsi
   const int wlen = s_hi - s_lo + 5;
   const bool use_smem = (s_lo <= s_hi) && wlen <= win_comp;
   if (use_smem)
-    for (int i = tid; i < ncomp * win_comp; i += kGapThreads) {
-      sWhi[i] = 0;
-      sWlo[i] = 0u;
+    for (int i = tid; i < ncomp * wlen; i += kGapThreads) {
+      const int si = (i / wlen) * win_comp + i % wlen;
+      sWhi[si] = 0;
+      sWlo[si] = 0u;
     }
   __syncthreads();
 
   const float *E3 = P.F[2].ptr;
   const float lower = P.m.lower[0], delta = P.m.delta[0];
+  // the members of the next slot are loaded while this one is pushed
+  struct Item {
+    float p1, x1, E, w;
+    uint32_t flag;
+  };
+  auto load_item = [&](int k, Item &m) {
+    const uint32_t c = cells[k];
+    if (c == AP_MAX_CELL || (int)c < g0 || (int)c >= n0 - g0) return;
+    const size_t idx = first + (size_t)k * kGapThreads + tid;
+    m.p1 = P.p.p1[idx];
+    m.x1 = P.p.x1[idx];
+    m.E = P.p.E[idx];
+    m.flag = P.p.flag[idx];
+    m.w = P.p.w[idx];
+  };
+  Item nxt{};
+  load_item(0, nxt);
 #pragma unroll 1
   for (int k = 0; k < kGapItems; ++k) {
+    const Item cur = nxt;
+    if (k + 1 < kGapItems) load_item(k + 1, nxt);
     const size_t idx = first + (size_t)k * kGapThreads + tid;
     const uint32_t c = cells[k];
     if (c == AP_MAX_CELL) continue;
@@ -108,10 +128,10 @@ __device__ void gap_chunk(const PushDepositParams &P, size_t ch, int *sWhi, unsi
       P.p.cell[idx] = AP_MAX_CELL;
       continue;
     }
-    float p1 = P.p.p1[idx];
-    const float x1 = P.p.x1[idx];
-    float gamma = P.p.E[idx];
-    const uint32_t flag = P.p.flag[idx];
+    float p1 = cur.p1;
+    const float x1 = cur.x1;
+    float gamma = cur.E;
+    const uint32_t flag = cur.flag;
     const int sp = ptc_type(flag);
     float beta = mesh_pos(lower, delta, (int)c, g0, x1);  // beta_phi(x) = x
     const float Dr = (x1 < 0.5f ? E3[c] * (0.5f + x1) + E3[c - 1] * (0.5f - x1)
@@ -137,7 +157,7 @@ __device__ void gap_chunk(const PushDepositParams &P, size_t ch, int *sWhi, unsi
     gamma = sqrtf(1.0f + p1 * p1 + beta * beta);
     P.p.E[idx] = gamma;
     if (!(flag & kFlagIgnoreCurrent)) {
-      const float weight = -P.charge[sp] * P.p.w[idx];
+      const float weight = -P.charge[sp] * cur.w;
       const int i0 = (dc1 == -1 ? -2 : -1), i1 = (dc1 == 1 ? 1 : 0);
       const bool rho = sp < ns;
       float djx = 0.0f;

@@ -92,17 +92,37 @@ __device__ void gr_chunk(const PushDepositParams &P, const GrK &G, size_t ch, in
   const int wlen = s_hi - s_lo + 5;
   const bool use_smem = (s_lo <= s_hi) && wlen <= win_comp;
   if (use_smem)
-    for (int i = tid; i < ncomp * win_comp; i += kGrThreads) {
-      sWhi[i] = 0;
-      sWlo[i] = 0u;
+    for (int i = tid; i < ncomp * wlen; i += kGrThreads) {
+      const int si = (i / wlen) * win_comp + i % wlen;
+      sWhi[si] = 0;
+      sWlo[si] = 0u;
     }
   __syncthreads();
 
   const float *E3 = P.F[2].ptr;
   const float lower = P.m.lower[0], delta = P.m.delta[0], inv_delta = P.m.inv_delta[0];
   const float dt = P.dt, a = G.a;
+  // the members of the next slot are loaded while this one is pushed
+  struct Item {
+    float p1, x1, E, w;
+    uint32_t flag;
+  };
+  auto load_item = [&](int k, Item &m) {
+    const uint32_t c = cells[k];
+    if (c == AP_MAX_CELL || (int)c < g0 || (int)c >= n0 - g0) return;
+    const size_t idx = first + (size_t)k * kGrThreads + tid;
+    m.p1 = P.p.p1[idx];
+    m.x1 = P.p.x1[idx];
+    m.E = P.p.E[idx];
+    m.flag = P.p.flag[idx];
+    m.w = P.p.w[idx];
+  };
+  Item nxt{};
+  load_item(0, nxt);
 #pragma unroll 1
   for (int k = 0; k < kGrItems; ++k) {
+    const Item cur = nxt;
+    if (k + 1 < kGrItems) load_item(k + 1, nxt);
     const size_t idx = first + (size_t)k * kGrThreads + tid;
     const uint32_t c = cells[k];
     if (c == AP_MAX_CELL) continue;
@@ -110,11 +130,11 @@ __device__ void gr_chunk(const PushDepositParams &P, const GrK &G, size_t ch, in
       P.p.cell[idx] = AP_MAX_CELL;
       continue;
     }
-    float p1 = P.p.p1[idx];
-    const float x1 = P.p.x1[idx];
-    float u0 = P.p.E[idx];
+    float p1 = cur.p1;
+    const float x1 = cur.x1;
+    float u0 = cur.E;
     float nx1 = 1.0f - x1;
-    const uint32_t flag = P.p.flag[idx];
+    const uint32_t flag = cur.flag;
     const int sp = ptc_type(flag);
     const float xi = mesh_pos(lower, delta, (int)c, g0, x1);
     const float rp = 1.0f + sqrtf(1.0f - a * a);
@@ -181,7 +201,7 @@ __device__ void gr_chunk(const PushDepositParams &P, const GrK &G, size_t ch, in
     P.p.E[idx] = u0;
     // deposit (:266-293): J1 through K1_j, Rho through K1, every step
     if (!(flag & kFlagIgnoreCurrent)) {
-      const float weight = -P.charge[sp] * P.p.w[idx];
+      const float weight = -P.charge[sp] * cur.w;
       const int i0 = (dc1 == -1 ? -2 : -1), i1 = (dc1 == 1 ? 1 : 0);
       const bool rho = sp < ns;
       float djx = 0.0f;
