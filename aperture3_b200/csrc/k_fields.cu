@@ -313,9 +313,9 @@ __global__ void k_filter_store(Geo G, const float *__restrict__ tmp, int tpitch,
 // exact, so the order of the adds does not matter; the only rounding is the
 // final conversion (int64 -> double is exact below 2^53, then one rounding
 // to FP32).
-__device__ __forceinline__ void finalize_cell(const Geo &G, const unsigned long long *a,
-                                              int acc_pitch, double inv, const Arr &out, int x,
-                                              int y) {
+__device__ __forceinline__ unsigned long long finalize_sum(const Geo &G,
+                                                           const unsigned long long *a,
+                                                           int acc_pitch, int x, int y) {
   int xi = -1, yi = -1;
   if (G.per0) {
     if (x >= G.g0 && x < 2 * G.g0) xi = x + G.r0;
@@ -331,26 +331,43 @@ __device__ __forceinline__ void finalize_cell(const Geo &G, const unsigned long 
     v += a[(size_t)yi * acc_pitch + x];
     if (xi >= 0) v += a[(size_t)yi * acc_pitch + xi];
   }
-  out(x, y) = (float)((double)(long long)v * inv);
+  return v;
 }
 
+// 2^-S for the formats' |S| <= 100.
+__device__ __forceinline__ double pow2_neg(int S) {
+  return __longlong_as_double((long long)(1023 - S) << 52);
+}
+
+struct FinalArrs {
+  Arr a[3 + AP_MAX_SPECIES];
+};
+
+// blockIdx.z the component; a thread rounds kFinalRows rows of one column, all
+// loads before the first store (one cell per thread and round took 59 us for
+// three components of 2048^2 cells, 151 MB).
+constexpr int kFinalRows = 4;
+
 __global__ void k_finalize(Geo G, const unsigned long long *__restrict__ acc, int acc_pitch,
-                           size_t acc_comp, const FixedFmt *fmt, int ncomp, Arr o0, Arr o1,
-                           Arr o2, Arr o3, Arr o4, Arr o5, Arr o6, Arr o7, Arr o8, Arr o9,
-                           Arr o10) {
+                           size_t acc_comp, const FixedFmt *fmt,
+                           const __grid_constant__ FinalArrs O) {
   const int rows = G.dim > 1 ? G.n1 : 1;
-  const size_t total = (size_t)G.n0 * rows;
-  const int comp = blockIdx.y;
-  if (comp >= ncomp) return;
-  Arr outs[11] = {o0, o1, o2, o3, o4, o5, o6, o7, o8, o9, o10};
-  const Arr out = outs[comp];
-  const unsigned long long *a = acc + comp * acc_comp;
-  const double inv = ldexp(1.0, -fmt->S);
-  for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < total;
-       t += (size_t)gridDim.x * blockDim.x) {
-    int x, y;
-    split_index(t, G.n0, x, y);
-    finalize_cell(G, a, acc_pitch, inv, out, x, y);
+  const int x = blockIdx.x * blockDim.x + threadIdx.x;
+  const int y0 = blockIdx.y * blockDim.y * kFinalRows + threadIdx.y;
+  if (x >= G.n0) return;
+  const Arr out = O.a[blockIdx.z];
+  const unsigned long long *a = acc + blockIdx.z * acc_comp;
+  const double inv = pow2_neg(fmt->S);
+  unsigned long long v[kFinalRows];
+#pragma unroll
+  for (int k = 0; k < kFinalRows; ++k) {
+    const int y = y0 + k * blockDim.y;
+    v[k] = y < rows ? finalize_sum(G, a, acc_pitch, x, y) : 0ull;
+  }
+#pragma unroll
+  for (int k = 0; k < kFinalRows; ++k) {
+    const int y = y0 + k * blockDim.y;
+    if (y < rows) out(x, y) = (float)((double)(long long)v[k] * inv);
   }
 }
 
@@ -437,10 +454,11 @@ __global__ void k_b1_finalize(const Run1D *__restrict__ runs, const uint32_t *__
     const int x = (int)(g - base[r]) * 256 + threadIdx.x;
     if (x >= R.n0) continue;
     const Geo G = geo1(R);
-    const double inv = ldexp(1.0, -R.fx->S);
+    const double inv = pow2_neg(R.fx->S);
     for (int comp = 0; comp < R.ncomp; ++comp) {
       const Arr out = farr(comp < 3 ? R.J[comp] : R.Rho[comp - 3]);
-      finalize_cell(G, R.acc + comp * R.acc_comp, R.n0, inv, out, x, 0);
+      const long long v = (long long)finalize_sum(G, R.acc + comp * R.acc_comp, R.n0, x, 0);
+      out(x, 0) = (float)((double)v * inv);
     }
   }
 }
@@ -704,17 +722,13 @@ cudaError_t launch_line_smooth_current(Ctx &c, const float *kj, const float *kr,
 
 cudaError_t launch_finalize_current(Ctx &c, int ncomp) {
   Geo G = make_geo(c);
-  Arr o[11];
-  for (int k = 0; k < 11; ++k) o[k] = Arr{nullptr, 0};
-  for (int k = 0; k < 3; ++k) o[k] = arr(c.fields.J[k]);
-  for (int s = 0; s < c.params.num_species && 3 + s < 11; ++s) o[3 + s] = arr(c.fields.Rho[s]);
-  const size_t total = (size_t)G.n0 * (G.dim > 1 ? G.n1 : 1);
-  int gx = (int)((total + 255) / 256);
-  if (gx > c.num_sms * 8) gx = c.num_sms * 8;
-  dim3 grid(gx, ncomp);
-  k_finalize<<<grid, 256, 0, c.stream>>>(G, c.acc, c.mesh.dims[0], c.acc_comp, c.fx_used, ncomp,
-                                         o[0], o[1],
-                                         o[2], o[3], o[4], o[5], o[6], o[7], o[8], o[9], o[10]);
+  FinalArrs O{};
+  for (int k = 0; k < 3; ++k) O.a[k] = arr(c.fields.J[k]);
+  for (int s = 0; s < c.params.num_species; ++s) O.a[3 + s] = arr(c.fields.Rho[s]);
+  const dim3 block = G.dim > 1 ? dim3(32, 8) : dim3(256, 1);
+  const int rows = (int)block.y * kFinalRows;
+  const dim3 grid((G.n0 + block.x - 1) / block.x, G.dim > 1 ? (G.n1 + rows - 1) / rows : 1, ncomp);
+  k_finalize<<<grid, block, 0, c.stream>>>(G, c.acc, c.mesh.dims[0], c.acc_comp, c.fx_used, O);
   c.launches++;
   return cudaGetLastError();
 }
