@@ -105,17 +105,30 @@ __device__ __forceinline__ void vay_push(float &p1, float &p2, float &p3, float 
   p3 = (up3 + B3 * ut * inv_gamma2 + (up1 * B2 - up2 * B1) / gamma) * s;
 }
 
-// vay_push followed by v = p / gamma, with the six quotients by the new gamma
-// through one reciprocal: the same bits. sigma + tt = 1 + up^2 and tt bound
-// every numerator from above; NaNs and numbers outside the bounds take the
-// plain divisions.
+// vay_push followed by v = p / gamma, gamma = sqrt(1 + p^2) on entry, with the
+// quotients by the old gamma and the six by the new one through a reciprocal
+// each: the same bits. gamma, sigma + tt = 1 + up^2 and tt bound every
+// numerator from above; NaNs and numbers outside the bounds take the plain
+// divisions.
 __device__ __forceinline__ void vay_push_v(float &p1, float &p2, float &p3, float &gamma,
                                            float E1, float E2, float E3, float B1, float B2,
                                            float B3, float &v1, float &v2, float &v3) {
-  const float up1 = p1 + 2.0f * E1 + (p2 * B3 - p3 * B2) / gamma;
-  const float up2 = p2 + 2.0f * E2 + (p3 * B1 - p1 * B3) / gamma;
-  const float up3 = p3 + 2.0f * E3 + (p1 * B2 - p2 * B1) / gamma;
   const float tt = B1 * B1 + B2 * B2 + B3 * B3;
+  float d1 = p2 * B3 - p3 * B2, d2 = p3 * B1 - p1 * B3, d3 = p1 * B2 - p2 * B1;
+  // |p| < gamma < 2^24, |B| < 2^15
+  if (gamma < 16777216.0f && tt < 1073741824.0f && !any_tiny(d1, d2, d3)) {
+    const SharedDiv by_gamma0(gamma);
+    d1 = by_gamma0(d1);
+    d2 = by_gamma0(d2);
+    d3 = by_gamma0(d3);
+  } else {
+    d1 = d1 / gamma;
+    d2 = d2 / gamma;
+    d3 = d3 / gamma;
+  }
+  const float up1 = p1 + 2.0f * E1 + d1;
+  const float up2 = p2 + 2.0f * E2 + d2;
+  const float up3 = p3 + 2.0f * E3 + d3;
   const float ut = up1 * B1 + up2 * B2 + up3 * B3;
   const float sigma = 1.0f + up1 * up1 + up2 * up2 + up3 * up3 - tt;
   const float inv_gamma2 = 2.0f / (sigma + sqrtf(sigma * sigma + 4.0f * (tt + ut * ut)));
@@ -128,7 +141,6 @@ __device__ __forceinline__ void vay_push_v(float &p1, float &p2, float &p3, floa
   // gamma < 2^24, |B| < 2^15, |up| < 2^31: numerators below 2^60
   const bool bounded = gamma < 16777216.0f && gamma > 0.5f && tt < 1073741824.0f &&
                        sigma < 4.6e18f;
-  float d1, d2, d3;
   if (bounded && !any_tiny(c1, c2, c3)) {
     d1 = by_gamma(c1);
     d2 = by_gamma(c2);

@@ -224,6 +224,9 @@ struct Ctx {
   uint2 *items = nullptr;
   size_t items_cap = 0;
   uint32_t item_len = 1;         // entries per item of the last list
+  const void *pd_kern = nullptr;  // last push / deposit variant, its blocks per SM
+  size_t pd_smem = 0;
+  int pd_per_sm = 0;
   size_t item_total = 0;         // in a batch: particles of all its 2D runs
   // per-chunk direction counts of the push / deposit (one-pass order update)
   uint32_t *chunk_count = nullptr;

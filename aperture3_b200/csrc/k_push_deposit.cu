@@ -174,7 +174,7 @@ struct TileGeom {
   static constexpr int JSZ = JX * JY;
   static constexpr int SP = CH + CH / 32;  // staged chunk, one pad word per 32
   static constexpr int HDR = 128;     // mbarrier, tile id, abort flag, counters
-  static constexpr size_t stage_bytes() { return 10 * 4 * SP + 2 * SP; }
+  static constexpr size_t stage_bytes() { return 10 * 4 * SP + (SP + 3) / 4 * 4; }
   static constexpr int NBUF = pipelined<CH>() ? 2 : 1;
   // double-buffered chunks: the order indices of the next two chunks
   static constexpr size_t order_bytes() { return NBUF == 2 ? 2 * 4 * CH : 0; }
@@ -431,8 +431,7 @@ __device__ __forceinline__ void push_deposit_tiles(const PushDepositParams &P0,
       uint32_t *s_cell = reinterpret_cast<uint32_t *>(stc + 7 * SP);
       uint32_t *s_flag = reinterpret_cast<uint32_t *>(stc + 8 * SP);
       uint32_t *s_idx = reinterpret_cast<uint32_t *>(stc + 9 * SP);
-      uint8_t *s_dir = reinterpret_cast<uint8_t *>(stc + 10 * SP);
-      uint8_t *s_mode = s_dir + SP;
+      uint8_t *s_dm = reinterpret_cast<uint8_t *>(stc + 10 * SP);  // direction, mode << 4
       // 3b. push + deposit: lane l of warp w takes element l*CH/32 + w*PER_THREAD + k
       for (int k = 0; k < PER_THREAD; ++k) {
         const int e = lane * (CH / 32) + warp * PER_THREAD + k;
@@ -447,8 +446,9 @@ __device__ __forceinline__ void push_deposit_tiles(const PushDepositParams &P0,
         const int c1 = (int)c - c2 * dims0;
         uint32_t dir = 4;
         uint8_t mode = 0;
-        const bool in_tile = (c != AP_MAX_CELL) && c1 >= x0 && c1 < x0 + TX && c2 >= y0 &&
-                             c2 < y0 + TY;
+        const int lx = c1 - x0, ly = c2 - y0;  // within the tile
+        const bool in_tile = c != AP_MAX_CELL && (unsigned)lx < (unsigned)TX &&
+                             (unsigned)ly < (unsigned)TY;
         if (!in_tile) {
           atomicAdd(&P.status->tile_faults, 1ull);
           dir = kDirGone;
@@ -482,8 +482,8 @@ __device__ __forceinline__ void push_deposit_tiles(const PushDepositParams &P0,
               acc += b.y;
               return acc * qm;
             };
-            const int i0 = Wx.base0 - (x0 - 1), i1 = c1 - x0;
-            const int j0 = (Wy.base0 - ys) * G::RX, j1 = (c2 - y0) * G::RX;
+            const int i0 = Wx.base0 - (x0 - 1), i1 = lx;
+            const int j0 = (Wy.base0 - ys) * G::RX, j1 = ly * G::RX;
             {
               const float4 r0 = sEB[j1 + i0], r1 = sEB[j1 + G::RX + i0];
               fe[0] = comp(make_float2(r0.x, r0.y), make_float2(r1.x, r1.y), Wx.w0, Wy.w1);
@@ -615,7 +615,7 @@ __device__ __forceinline__ void push_deposit_tiles(const PushDepositParams &P0,
                   J3{sJhi + 2 * G::JSZ, sJlo + 2 * G::JSZ};
               const Acc32 R{sJhi + (3 + sp) * G::JSZ, sJlo + (3 + sp) * G::JSZ};
               const bool rho = kRho && P.do_rho && sp < P.num_species;
-              const int o = (c2 + jb - jy0) * G::JX + (c1 + ib - jx0);
+              const int o = (ly + jb + 2) * G::JX + (lx + ib + 2);
               {
                 const float h = 0.5f * wsc;
                 // the cumulative sums from either end (the weights add up to 1)
@@ -707,19 +707,18 @@ __device__ __forceinline__ void push_deposit_tiles(const PushDepositParams &P0,
           }
           // move + wrap through periodic sides (send_particles semantics)
           int c1n = c1 + dc1, c2n = c2 + dc2;
+          // past the upper end of the bulk: the next tile, also from a tile
+          // that the end cuts short
+          const bool over1 = c1n >= dims0 - g0, over2 = c2n >= dims1 - g1;
           bool keep = !far;
           keep = keep && wrap_coord(c1n, g0, dims0, P.m.red[0], P.periodic[0]);
           keep = keep && wrap_coord(c2n, g1, dims1, P.m.red[1], P.periodic[1]);
           uint32_t ncell = AP_MAX_CELL;
           if (keep) {
             ncell = (uint32_t)(c1n + c2n * dims0);
-            int dtx = (c1n - g0) / TX - tix;
-            int dty = (c2n - g1) / TY - tiy;
-            if (dtx > 1) dtx = -1;
-            if (dtx < -1) dtx = 1;
-            if (dty > 1) dty = -1;
-            if (dty < -1) dty = 1;
-            dir = (uint32_t)((dty + 1) * 3 + (dtx + 1));
+            const int dtx = lx + dc1 < 0 ? 0 : (lx + dc1 >= TX || over1 ? 2 : 1);
+            const int dty = ly + dc2 < 0 ? 0 : (ly + dc2 >= TY || over2 ? 6 : 3);
+            dir = (uint32_t)(dty + dtx);
             if constexpr (kLS) {
               // ptc_outflow (ptc_updater_logsph.cu:440-455)
               if (!(flag & kFlagIgnoreEM) && c1n > P.ls_outflow_c1) {
@@ -747,8 +746,7 @@ __device__ __forceinline__ void push_deposit_tiles(const PushDepositParams &P0,
             mode |= kWriteMom;
           }
         }
-        s_dir[s] = (uint8_t)dir;
-        s_mode[s] = mode;
+        s_dm[s] = (uint8_t)(dir | (uint32_t)mode << 4);
         // direction counts: one add per warp for the particles that stay in
         // the tile (nearly all), one per particle for the rest
         const unsigned act = __activemask();
@@ -769,7 +767,7 @@ __device__ __forceinline__ void push_deposit_tiles(const PushDepositParams &P0,
         const int e = tid + k * kThreads2D;
         if (e < nch) {
           const int s = spos(e);
-          const uint8_t mode = s_mode[s];
+          const uint32_t dm = s_dm[s], mode = dm >> 4;
           const uint32_t idx = s_idx[s];
           if (P.cout.x1) {
             // compaction: every member to its tile-list position
@@ -785,7 +783,7 @@ __device__ __forceinline__ void push_deposit_tiles(const PushDepositParams &P0,
             P.cout.cell[q] = s_cell[s];
             P.cout.flag[q] = s_flag[s];
             P.cout_id[q] = P.id[idx];
-            P.dir[base + c0 + e] = s_dir[s];
+            P.dir[base + c0 + e] = (uint8_t)(dm & 15u);
             continue;
           }
           if (mode & kWritePos) {
@@ -801,7 +799,7 @@ __device__ __forceinline__ void push_deposit_tiles(const PushDepositParams &P0,
             P.p.E[idx] = s_w[s];
           }
           if (kLS && (mode & kWriteFlag)) P.p.flag[idx] = s_flag[s];
-          P.dir[base + c0 + e] = s_dir[s];
+          P.dir[base + c0 + e] = (uint8_t)(dm & 15u);
         }
       }
       if (G::NBUF == 2) cp_async_wait_group<0>();  // the next chunk and order indices
@@ -878,19 +876,36 @@ __device__ __forceinline__ float interp_1d_global(const FieldArr &f, const Weigh
   return acc;
 }
 
-// Warp-collective deposit of one node into the 1D window (every lane of the
-// warp calls it; `act` lanes contribute a1 to J1 at window offset o + 1 and
-// a2, a3 to J2, J3 at o). In a cell-sorted run neighbouring lanes hold
-// particles of the same cell, so their atomics would all hit one address:
-// when more than kAgg1D lanes are active but they touch at most kAgg1D
-// distinct offsets, each offset's fixed-point words are summed across its
-// lanes (integer sums, so the result is the same bits) and one lane adds
-// them; a few active lanes add directly.
+// Warp-collective deposit of a warp's particles into the 1D window. In a
+// cell-sorted run neighbouring lanes hold particles of the same cell, so their
+// atomics would all hit one address: when the lanes touch at most kAgg1D
+// distinct first nodes, each node's fixed-point words are summed across the
+// lanes that share it (integer sums, so the result is the same bits) and one
+// lane adds them; a few active lanes, and nodes of many cells, add directly.
 constexpr int kAgg1D = 4;
 
-__device__ __forceinline__ void deposit_1d_node(bool act, int o, float a1, float a2, float a3,
-                                                int *hi, unsigned *lo, int win_comp,
-                                                float scale, int L) {
+// The lanes that share a first node: found once per particle for its two or
+// three nodes.
+struct Groups1D {
+  unsigned leaders;  // lowest lane of each group
+  bool few;          // at most kAgg1D groups
+};
+
+__device__ __forceinline__ Groups1D groups_1d(bool act, int o) {
+  const int lane = threadIdx.x & 31;
+  const unsigned key = act ? (unsigned)o : (0x80000000u | (unsigned)lane);
+  const unsigned peers = __match_any_sync(0xffffffffu, key);
+  Groups1D g;
+  g.leaders = __ballot_sync(0xffffffffu, act && lane == __ffs(peers) - 1);
+  g.few = __popc(g.leaders) <= kAgg1D;
+  return g;
+}
+
+// One node (every lane of the warp calls it): `act` lanes contribute a1 to J1
+// at window offset o + 1 and a2, a3 to J2, J3 at o; g groups the offsets.
+__device__ __forceinline__ void deposit_1d_node(const Groups1D &g, bool act, int o, float a1,
+                                                float a2, float a3, int *hi, unsigned *lo,
+                                                int win_comp, float scale, int L) {
   const unsigned am = __ballot_sync(0xffffffffu, act);
   if (am == 0u) return;
   const int lane = threadIdx.x & 31;
@@ -904,21 +919,8 @@ __device__ __forceinline__ void deposit_1d_node(bool act, int o, float a1, float
     l[c] = (unsigned)X & mask;
   }
   const int dst[3] = {o + 1, win_comp + o, 2 * win_comp + o};
-  if (__popc(am) <= kAgg1D) {  // few lanes (the outer nodes of crossing particles): add directly
-    if (act) {
-#pragma unroll
-      for (int c = 0; c < 3; ++c) {
-        atomicAdd(hi + dst[c], (int)h[c]);
-        atomicAdd(lo + dst[c], l[c]);
-      }
-    }
-    return;
-  }
-  const unsigned key = act ? (unsigned)o : (0x80000000u | (unsigned)lane);
-  const unsigned peers = __match_any_sync(0xffffffffu, key);
-  const unsigned leaders = __ballot_sync(0xffffffffu, act && lane == __ffs(peers) - 1);
-  if (__popc(leaders) <= kAgg1D) {
-    for (unsigned m = leaders; m != 0u; m &= m - 1u) {
+  if (g.few && __popc(am) > kAgg1D) {
+    for (unsigned m = g.leaders; m != 0u; m &= m - 1u) {
       const int ld = __ffs(m) - 1;
       const int ko = __shfl_sync(0xffffffffu, o, ld);  // every lane takes part
       const bool in = act && o == ko;
@@ -1098,6 +1100,7 @@ __device__ __forceinline__ void push_deposit_1d_chunk(const PushDepositParams &P
       // a cell crossing), in the reference's order
       const int i0 = (d_dc1 == -1 ? -2 : -1), i1 = (d_dc1 == 1 ? 1 : 0);
       float djx = 0.0f;
+      const Groups1D groups = groups_1d(dep, i0 + d_c1 - wlo);
 #pragma unroll
       for (int j = 0; j < 3; ++j) {
         const int i = i0 + j;
@@ -1114,7 +1117,8 @@ __device__ __forceinline__ void push_deposit_1d_chunk(const PushDepositParams &P
           a3 = weight * d_v3 * val1;
         }
         if (use_smem) {
-          deposit_1d_node(act, off - wlo, a1, a2, a3, sWhi, sWlo, win_comp, fscale, fx.L);
+          deposit_1d_node(groups, act, off - wlo, a1, a2, a3, sWhi, sWlo, win_comp, fscale,
+                          fx.L);
           if (act && kRho && P.do_rho && d_sp < P.num_species) {
             const Acc32 W{sWhi, sWlo};
             add_fixed(W, (3 + d_sp) * win_comp + off - wlo, weight * sx1, fscale, fx.L);
@@ -1195,14 +1199,20 @@ cudaError_t launch_2d_tiles(Ctx &c, const PushDepositParams &P) {
   const int nrho = P.do_rho ? P.num_species : 0;
   const size_t smem = G::smem_bytes(nrho, kLS);  // the queue was cleared with the status
   auto run = [&](auto kern) -> cudaError_t {
-    cudaError_t err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           (int)smem);
-    if (err != cudaSuccess) return err;
-    int per_sm = 0;
-    err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kThreads2D, smem);
-    if (err != cudaSuccess) return err;
-    if (per_sm < 1) return cudaErrorInvalidConfiguration;
-    size_t grid = (size_t)c.num_sms * per_sm;
+    // blocks per SM of the variant, asked for when the context's variant changes
+    if (c.pd_kern != reinterpret_cast<const void *>(kern) || c.pd_smem != smem) {
+      cudaError_t err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             (int)smem);
+      if (err != cudaSuccess) return err;
+      int per_sm = 0;
+      err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kThreads2D, smem);
+      if (err != cudaSuccess) return err;
+      if (per_sm < 1) return cudaErrorInvalidConfiguration;
+      c.pd_kern = reinterpret_cast<const void *>(kern);
+      c.pd_smem = smem;
+      c.pd_per_sm = per_sm;
+    }
+    size_t grid = (size_t)c.num_sms * c.pd_per_sm;
     const size_t items = P.t.ntiles + (c.number - c.store_base) / c.item_len;  // at most
     if (grid > items) grid = items;
     if (grid < 1) grid = 1;
