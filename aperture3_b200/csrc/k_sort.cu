@@ -688,10 +688,10 @@ int ensure_scratch(Ctx &c, size_t n) {
   return AP_OK;
 }
 
-// After a compaction: the slots after the live ones are empty.
+// After a compaction: the slots after the live ones (none, or a few that left
+// the grid) are empty.
 __global__ void k_compact_tail(const uint32_t *live, uint32_t *cell, size_t n) {
-  const uint32_t m = *live;
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n;
+  for (size_t i = *live + blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n;
        i += (size_t)gridDim.x * blockDim.x)
     cell[i] = AP_MAX_CELL;
 }
