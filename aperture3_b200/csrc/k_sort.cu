@@ -486,23 +486,13 @@ __global__ void __launch_bounds__(kScanThreads)
 }
 static_assert(kScanThreads == 1024, "one warp scans the 32 warp sums");
 
-// dst[i] = src[perm[i]], one entry per thread and round: for members larger
-// than the L2, whose sources must stay close together in it.
-template <typename T>
-__global__ void k_gather(const T *__restrict__ src, const uint32_t *__restrict__ perm, size_t n,
-                         T *__restrict__ dst) {
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n;
-       i += (size_t)gridDim.x * blockDim.x)
-    dst[i] = src[perm[i]];
-}
-
-// The same with four consecutive entries per thread: the permutation and the
-// result move 16 bytes at a time and four gathers are in flight. The first
+// dst[i] = src[perm[i]], four consecutive entries per thread: the permutation
+// and the result move 16 bytes at a time and four gathers are in flight. The first
 // `head` entries, up to dst's 16-byte boundary, go one by one; with a head the
 // permutation's words are read singly.
 template <typename T>
-__global__ void k_gather4(const T *__restrict__ src, const uint32_t *__restrict__ perm, size_t n,
-                          T *__restrict__ dst, int head) {
+__global__ void k_gather(const T *__restrict__ src, const uint32_t *__restrict__ perm, size_t n,
+                         T *__restrict__ dst, int head) {
   const size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
   const size_t stride = (size_t)gridDim.x * blockDim.x * 4;
   if (t < (size_t)head && t < n) dst[t] = src[perm[t]];
@@ -572,16 +562,16 @@ cudaError_t gather_member(Ctx &c, const void *src, const uint32_t *perm, size_t 
                           void *dst) {
   const int off = (int)(reinterpret_cast<uintptr_t>(dst) & 15u);
   const int head = off ? (16 - off) / bytes : 0;  // an 8-byte member starts at 0 or 8
-  // four entries per thread while the member fits the 126 MB L2: 8.4 M 4-byte
-  // members 32 -> 19 us, 16.8 M 62 -> 55 us; past it their sources, in a store
-  // in tile order, spread too far: 67 M 264 -> 286 us, 8-byte 339 -> 635 us
-  const bool four = n * (size_t)bytes <= (size_t)128 << 20;
+  // a member that fits the 126 MB L2 takes 16 blocks per SM (8.4 M 4-byte
+  // entries: 32 us one per thread, 19 us so); a larger one four, which keeps
+  // the sources in flight of a store in tile order close together (all eleven
+  // members of 67 M: 2.98 ms one per thread, 3.2 ms with 16 blocks)
+  const int blocks = n * (size_t)bytes <= (size_t)128 << 20 ? 16 : 4;
+  int g = grid_for(c, (n + 3) / 4, 256);
+  if (g > c.num_sms * blocks) g = c.num_sms * blocks;
   auto run = [&](auto *s, auto *d) {
     using T = std::remove_pointer_t<decltype(d)>;
-    if (four)
-      k_gather4<T><<<grid_for(c, (n + 3) / 4, 256), 256, 0, c.stream>>>(s, perm, n, d, head);
-    else
-      k_gather<T><<<grid_for(c, n, 256), 256, 0, c.stream>>>(s, perm, n, d);
+    k_gather<T><<<g, 256, 0, c.stream>>>(s, perm, n, d, head);
   };
   if (bytes == 8)
     run(static_cast<const uint64_t *>(src), static_cast<uint64_t *>(dst));
