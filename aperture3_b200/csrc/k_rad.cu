@@ -288,18 +288,14 @@ __device__ __forceinline__ bool may_emit(const RadK &K, float gamma) {
   return true;
 }
 
-// check_emit_photon (default :13-17; pulsar :26-53).
-__device__ bool check_emit(const RadK &K, const PtcK &p, size_t tid, uint32_t cell,
-                           const float u[4]) {
-  const float gamma = p.E[tid];
-  if (K.model == AP_RAD_DEFAULT) return gamma > K.gamma_thr;
-  if (K.model == AP_RAD_GR1D) return check_emit_gr(K, p, tid, cell, u);
-  if (K.model == AP_RAD_GAP1D) return check_emit_gap(K, p, tid, u);
-  const int c1 = c1_of(K.m, cell), c2 = c2_of(K.m, cell);
-  const float r = expf(mpos(K.m, 0, c1, p.x1[tid]));
+// check_emit_photon of the pulsar lab (:26-53) for a particle whose members are
+// loaded, u0 its first draw.
+__device__ __forceinline__ bool check_emit_pulsar(const RadK &K, float gamma, float x1, float x2,
+                                                  int c1, int c2, float u0) {
+  const float r = expf(mpos(K.m, 0, c1, x1));
   if (r > 0.6f / K.omega) return false;
   if ((double)r < 1.05) return false;
-  const float theta = mpos(K.m, 1, c2, p.x2[tid]);
+  const float theta = mpos(K.m, 1, c2, x2);
   const float num = K.delta_t * gamma;
   const float en = K.e_curv * gamma * gamma * gamma;
   {
@@ -312,15 +308,15 @@ __device__ bool check_emit(const RadK &K, const PtcK &p, size_t tid, uint32_t ce
     if (sn > 1.0e-4f) {
       const float rf = r * (t * sqrtf(t)) / (3.0f * sn * (1.0f + c * c));
       const float rate = num / (K.l_curv * rf), eph = en / rf;
-      if (rf < 0.9999f || u[0] > rate * 1.0001f || eph < 2.1f * 0.9999f) return false;
-      if (rf > 1.0001f && u[0] < rate * 0.9999f && eph > 2.1f * 1.0001f) return true;
+      if (rf < 0.9999f || u0 > rate * 1.0001f || eph < 2.1f * 0.9999f) return false;
+      if (rf > 1.0001f && u0 < rate * 0.9999f && eph > 2.1f * 1.0001f) return true;
     }
   }
   const float rc = rho_c(r, theta);
   if (rc < 1.0f) return false;
   const float rate = num / (K.l_curv * rc);
   const float Eph = en / rc;
-  return u[0] < rate && Eph > 2.1f;
+  return u0 < rate && Eph > 2.1f;
 }
 
 // emit_photon (default :19-63; pulsar :55-131): the parent loses the photon
@@ -571,8 +567,27 @@ struct WarpList {
   uint8_t hit[kRadThreads / 32][32 * kRadPer];   // the test's answer per slot
 };
 
-// Lists the slots with want[k] set and runs test(index in the store) on each;
-// bit k of the result: slot k of this lane passed.
+// Asynchronous copy of one 4- or 8-byte member into shared memory: the members
+// that the emission test of the listed slots needs arrive together, without
+// holding registers, before the list is worked through (each round waited for
+// its own loads otherwise: 126 us for the mark of 6.3 M slots, 105 us so; held
+// in registers they cost occupancy, 167 us). The conversion test, which goes on
+// to load the fields anyway, gains nothing from it (90 and 93 us).
+template <typename T>
+__device__ __forceinline__ void fetch_member(T *dst, const T *src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(
+                   static_cast<uint32_t>(__cvta_generic_to_shared(dst))),
+               "l"(src), "n"(sizeof(T))
+               : "memory");
+}
+__device__ __forceinline__ void fetched() {
+  asm volatile("cp.async.wait_all;" ::: "memory");
+  __syncwarp();
+}
+
+// Lists the slots with want[k] set and runs test(index in the store, place
+// among the warp's slots) on each; bit k of the result: slot k of this lane
+// passed.
 template <class Test>
 __device__ __forceinline__ uint32_t test_listed(WarpList &L, size_t first_of_chunk,
                                                 const bool want[kRadPer], Test &&test) {
@@ -590,7 +605,7 @@ __device__ __forceinline__ uint32_t test_listed(WarpList &L, size_t first_of_chu
   for (int r = lane; r < n; r += 32) {
     const int e = L.slot[warp][r];
     const size_t idx = first_of_chunk + (size_t)(e >> 5) * kRadThreads + warp * 32 + (e & 31);
-    if (test(idx)) L.hit[warp][e] = 1;
+    if (test(idx, e)) L.hit[warp][e] = 1;
   }
   __syncwarp();
   uint32_t em = 0;
@@ -600,10 +615,17 @@ __device__ __forceinline__ uint32_t test_listed(WarpList &L, size_t first_of_chu
   return em;
 }
 
+struct EmitRec {
+  uint64_t id;
+  float x1, x2, gamma;
+  uint32_t cell;
+};
+
 __global__ void __launch_bounds__(kRadThreads)
     k_rad_emit_mark(RadK K, PtcK p, const uint64_t *ids, size_t number, uint8_t *mark,
                     uint32_t *counts, uint32_t nchunks) {
   __shared__ WarpList L;
+  __shared__ EmitRec s_rec[kRadChunk];
   for (uint32_t ch = blockIdx.x; ch < nchunks; ch += gridDim.x) {
     const size_t first = (size_t)ch * kRadChunk + threadIdx.x;
     uint32_t cell[kRadPer], flag[kRadPer];
@@ -623,11 +645,33 @@ __global__ void __launch_bounds__(kRadThreads)
       want[k] = cell[k] != AP_MAX_CELL && bulk_cell(K.m, cell[k], c1, c2) &&
                 (flag[k] >> 29) != 2u && may_emit(K, gam[k]);
     }
-    const uint32_t em = test_listed(L, (size_t)ch * kRadChunk, want, [&](size_t idx) {
+    if (K.model == AP_RAD_PULSAR) {
+#pragma unroll
+      for (int k = 0; k < kRadPer; ++k)
+        if (want[k]) {
+          const size_t idx = first + (size_t)k * kRadThreads;
+          EmitRec &r = s_rec[threadIdx.x + k * kRadThreads];
+          fetch_member(&r.id, ids + idx);
+          fetch_member(&r.x1, p.x1 + idx);
+          fetch_member(&r.x2, p.x2 + idx);
+          r.gamma = gam[k];
+          r.cell = cell[k];
+        }
+      fetched();
+    }
+    const uint32_t em = test_listed(L, (size_t)ch * kRadChunk, want, [&](size_t idx, int) {
       if (K.model == AP_RAD_DEFAULT) return true;  // may_emit is its whole test
       float u[4];
+      if (K.model == AP_RAD_PULSAR) {
+        const EmitRec &r = s_rec[idx - (size_t)ch * kRadChunk];
+        int c1, c2;
+        bulk_cell(K.m, r.cell, c1, c2);
+        uniforms(K, 1u, r.id, u);
+        return check_emit_pulsar(K, r.gamma, r.x1, r.x2, c1, c2, u[0]);
+      }
       uniforms(K, 1u, ids[idx], u);
-      return check_emit(K, p, idx, p.cell[idx], u);
+      return K.model == AP_RAD_GR1D ? check_emit_gr(K, p, idx, p.cell[idx], u)
+                                    : check_emit_gap(K, p, idx, u);
     });
 #pragma unroll
     for (int k = 0; k < kRadPer; ++k) {
@@ -688,7 +732,7 @@ __global__ void __launch_bounds__(kRadThreads)
       int c1, c2;
       want[k] = cell[k] != AP_MAX_CELL && bulk_cell(K.m, cell[k], c1, c2);
     }
-    const uint32_t em = test_listed(L, (size_t)ch * kRadChunk, want, [&](size_t idx) {
+    const uint32_t em = test_listed(L, (size_t)ch * kRadChunk, want, [&](size_t idx, int) {
       if (K.model == AP_RAD_DEFAULT) return ph.path[idx] <= 0.0f;
       const uint32_t c = ph.cell[idx];
       if (K.model == AP_RAD_PULSAR) {
