@@ -41,7 +41,12 @@ cudaError_t alloc_control(Ctx &c) {
   cudaFree(c.status);
   c.status = nullptr;
   c.queue = c.dir_count = nullptr;
-  const size_t bytes = kControlHead + sizeof(uint32_t) * ((size_t)c.tiles.ntiles * 10 + 16);
+  c.acc = nullptr;
+  c.acc_comp = (size_t)c.mesh.dims[0] * c.mesh.dims[1] * c.mesh.dims[2];
+  const size_t counts = c.mk.dim == 2 ? sizeof(uint32_t) * ((size_t)c.tiles.ntiles * 10 + 16) : 0;
+  c.acc_offset = (kControlHead + counts + 255) / 256 * 256;
+  const size_t bytes =
+      c.acc_offset + sizeof(unsigned long long) * c.acc_comp * (3 + c.params.num_species);
   unsigned char *b = nullptr;
   cudaError_t e = cudaMalloc(reinterpret_cast<void **>(&b), bytes);
   if (e != cudaSuccess) return e;
@@ -49,7 +54,13 @@ cudaError_t alloc_control(Ctx &c) {
   c.status = reinterpret_cast<DevStatus *>(b);
   c.queue = reinterpret_cast<uint32_t *>(b + sizeof(DevStatus));
   c.dir_count = reinterpret_cast<uint32_t *>(b + kControlHead);
-  return cudaMemset(b, 0, bytes);
+  c.acc = reinterpret_cast<unsigned long long *>(b + c.acc_offset);
+  return cudaMemset(b, 0, c.acc_offset);
+}
+
+cudaError_t clear_control(Ctx &c, int ncomp) {
+  return cudaMemsetAsync(c.status, 0,
+                         c.acc_offset + sizeof(unsigned long long) * c.acc_comp * ncomp, c.stream);
 }
 
 }  // namespace apb
@@ -343,7 +354,6 @@ AP_API int ap_ctx_destroy(ap_ctx *c) {
   cudaFree(c->pair_chunks);
   cudaFree(c->pstate);
   if (c->pstate_host) cudaFreeHost(c->pstate_host);
-  cudaFree(c->acc);
   cudaFree(c->fx_used);
   cudaFree(c->n_max);
   cudaFree(c->wmax);
@@ -399,11 +409,6 @@ AP_API int ap_bind_fields(ap_ctx *c, const ap_fields *f) {
   c->fields_bound = true;
   c->rho_is_zero = false;
   c->use_tma = setup_tensor_maps(*c);
-  if (!c->acc) {
-    c->acc_comp = (size_t)m.dims[0] * m.dims[1] * m.dims[2];
-    AP_TRY(cudaMalloc(&c->acc, sizeof(unsigned long long) * c->acc_comp *
-                                   (3 + c->params.num_species)));
-  }
   if (!c->tmp_j) {
     size_t pitch = sizeof(float) * (size_t)m.dims[0];
     AP_TRY(cudaMalloc(&c->tmp_j, pitch * (size_t)m.dims[1] * m.dims[2]));
@@ -501,10 +506,8 @@ int update_particles_gap(Ctx *c, double dt, uint32_t step) {
   const int bl = !pr.periodic[0], bu = !pr.periodic[0];  // is_boundary(0), (1)
   int ph = phase_begin(c, kPhFinalize);
   // J and Rho are zeroed (:227-230); the finalize writes every component
-  AP_TRY(cudaMemsetAsync(c->acc, 0, sizeof(unsigned long long) * c->acc_comp * ncomp,
-                         c->stream));
+  AP_TRY(clear_control(*c, ncomp));
   if (!c->scale_valid) AP_TRY(launch_fixed_scale(*c));
-  AP_TRY(cudaMemsetAsync(c->status, 0, sizeof(DevStatus), c->stream));
   // E3 = E1, smoothed current_smoothing times through E2 (:232-240)
   float *E1 = c->fields.E[0].ptr, *E2 = c->fields.E[1].ptr, *E3 = c->fields.E[2].ptr;
   const bool fits = line_smooth_fits(*c);
@@ -585,10 +588,8 @@ int update_particles_gr(Ctx *c, double dt, uint32_t step) {
   const float *K1 = coef_array(*c, AP_GR_K1).ptr, *K1j = coef_array(*c, AP_GR_K1_J).ptr;
   int ph = phase_begin(c, kPhFinalize);
   // J and Rho are zeroed (:423-426); the finalize writes every component
-  AP_TRY(cudaMemsetAsync(c->acc, 0, sizeof(unsigned long long) * c->acc_comp * ncomp,
-                         c->stream));
+  AP_TRY(clear_control(*c, ncomp));
   if (!c->scale_valid) AP_TRY(launch_fixed_scale(*c));
-  AP_TRY(cudaMemsetAsync(c->status, 0, sizeof(DevStatus), c->stream));
   // E3 = E1, smoothed current_smoothing times through E2 with K1_j (:428-435)
   float *E1 = c->fields.E[0].ptr, *E2 = c->fields.E[1].ptr, *E3 = c->fields.E[2].ptr;
   const bool fits = line_smooth_fits(*c);
@@ -683,22 +684,15 @@ int update_prepare(Ctx *c, double dt, uint32_t step, PushDepositParams &P, bool 
   const int ncomp = 3 + (do_rho ? pr.num_species : 0);
   const bool ls = c->coord == 1;
   int ph = phase_begin(c, kPhFinalize);
-  if (!batched)
-    AP_TRY(cudaMemsetAsync(c->acc, 0, sizeof(unsigned long long) * c->acc_comp * ncomp,
-                           c->stream));
+  // the accumulators and, in the same block, the status, the queue and the
+  // direction counts the 2D push adds to
+  if (!batched) AP_TRY(clear_control(*c, ncomp));
   if (!c->scale_valid) AP_TRY(launch_fixed_scale(*c));
   // Rho keeps the zeros of the last step without charge deposition
   if (!do_rho && !ls && !c->rho_is_zero) {
     for (int s = 0; s < pr.num_species; ++s) AP_TRY(launch_zero(*c, c->fields.Rho[s]));
     c->rho_is_zero = true;
   }
-  // status, queue and, in 2D, the direction counts the push adds to
-  if (!batched)
-    AP_TRY(cudaMemsetAsync(c->status, 0,
-                           c->mk.dim == 2 ? kControlHead + sizeof(uint32_t) * 10 *
-                                                               (size_t)c->tiles.ntiles
-                                          : kControlHead,
-                           c->stream));
   // continuity check: rho(t) of the previous update, before it is replaced
   c->cont_snap = false;
   if (c->cont_on && !batched && !ls && do_rho && c->last_rho_step == (long long)step - 1) {

@@ -212,9 +212,7 @@ struct Ctx {
   int cur = 0;
   bool order_valid = false;
   uint8_t *dir = nullptr;
-  // one block, cleared by one memset per update: the status, the work queue
-  // and the per-tile direction counts
-  uint32_t *dir_count = nullptr;
+  uint32_t *dir_count = nullptr;  // in the control block
   uint32_t *grp_off = nullptr;
   uint32_t *newcount = nullptr;  // per-tile population after the step
   uint32_t *queue = nullptr;
@@ -243,9 +241,11 @@ struct Ctx {
   uint32_t *cell_count = nullptr;  // ncells + 1 entries (tile-local sort)
   uint32_t *sort_max = nullptr;    // device: largest cell population (tile-local sort)
 
-  // fixed-point current / charge accumulators (3 + num_species components)
+  // fixed-point current / charge accumulators (3 + num_species components),
+  // in the control block
   unsigned long long *acc = nullptr;
   size_t acc_comp = 0;
+  size_t acc_offset = 0;        // of acc in the control block
   FixedFmt *fx_used = nullptr;  // device: format of the last deposit
   uint32_t *n_max = nullptr;    // device: largest tile population, number of work items, item length
   float *wmax = nullptr;        // device: max |weight| over the bound particles
@@ -465,9 +465,12 @@ int fill_run1d(Ctx *c, double dt, uint32_t step, Run1D &d);
 
 int ctx_check_status(Ctx *c);
 
-// The control block of a context: status, queue, direction counts of ntiles
-// tiles. Allocates (or replaces) it and clears it.
+// The control block of a context: status, queue, direction counts of the tiles
+// (2D), fixed-point accumulators. alloc_control allocates (or replaces) it;
+// clear_control clears it for an update of ncomp accumulator components, one
+// memset.
 cudaError_t alloc_control(Ctx &c);
+cudaError_t clear_control(Ctx &c, int ncomp);
 constexpr size_t kControlHead = 64;  // bytes before the direction counts
 
 // One persistent push / deposit launch over the tiles of several 2D
