@@ -39,7 +39,8 @@ __device__ __forceinline__ float cic(float dx) {
 // exact: the distances are f, 1 - f, |0.5 - f| and so on, so the weights are
 // 1 - f and f (stagger 1), and 0.5 -+ f or 1.5 - f, f - 0.5 (stagger 0), the
 // same bits as the reference's fl(1 - |node - xc|) in a third of the
-// instructions.
+// instructions. Offsets outside [0, 1], NaNs and cells further out take the
+// expressions themselves.
 struct Weights1D {
   int base0;       // first node for stagger 0 (c-1 or c)
   float w0[2];     // stagger-0 weights of nodes base0, base0 + 1
@@ -49,13 +50,24 @@ struct Weights1D {
 __device__ __forceinline__ Weights1D weights_1d(float rel, int c) {
   Weights1D W;
   const float fc = (float)c;
-  const float f = (rel + fc) - fc;
-  W.w1[0] = 1.0f - f;
-  W.w1[1] = f;
-  const bool low = f < 0.5f;
-  W.base0 = low ? c - 1 : c;
-  W.w0[0] = (low ? 0.5f : 1.5f) - f;
-  W.w0[1] = f + (low ? 0.5f : -0.5f);
+  const float xc = rel + fc;
+  const float f = xc - fc;
+  // one test of the bits: f is in [0, 1] and no NaN
+  if (__float_as_uint(f) <= __float_as_uint(1.0f) && c < (1 << 22)) {
+    const bool low = f < 0.5f;
+    W.base0 = low ? c - 1 : c;
+    W.w1[0] = 1.0f - f;
+    W.w1[1] = f;
+    W.w0[0] = (low ? 0.5f : 1.5f) - f;
+    W.w0[1] = f + (low ? 0.5f : -0.5f);
+  } else {
+    W.base0 = xc < fc + 0.5f ? c - 1 : c;
+    const float fb = (float)W.base0;
+    W.w1[0] = cic(((float)(c - 1) + 1.0f) - xc);
+    W.w1[1] = cic((fc + 1.0f) - xc);
+    W.w0[0] = cic((fb + 0.5f) - xc);
+    W.w0[1] = cic(((float)(W.base0 + 1) + 0.5f) - xc);
+  }
   return W;
 }
 
