@@ -6,16 +6,18 @@
 //
 // 2D design: the particles are kept in a stable tile order (one list of
 // slot indices per tile of TX x TY cells, maintained by a counting sort each
-// step). A persistent CTA takes tiles from a queue; for each tile it
-//   1. stages the E/B tile plus a one-cell halo into shared memory with six
-//      TMA 2D tiled loads (no multicast) completing on an mbarrier,
+// step). A persistent CTA takes work items from a queue, an item being a
+// tile's list or a part of a long one; for each item it
+//   1. brings the E/B tile plus a one-cell halo into shared memory with six
+//      TMA 2D tiled loads (no multicast) completing on an mbarrier, and lays
+//      it out as one record per cell (wide loads in the gather),
 //   2. zeroes a shared-memory J (and Rho) tile with a two-cell halo,
-//   3. walks the tile's list in chunks of CH particles: a coalesced load
-//      stages the chunk's records in shared memory, each warp then pushes
-//      and deposits 32 particles that sit CH/32 places apart in the list
-//      (in a cell-sorted list that puts the lanes of a warp in different
-//      cells, so their current updates do not collide), and a coalesced
-//      store writes the chunk back,
+//   3. walks the item's list in chunks of CH particles, the next chunk's
+//      records in flight (cp.async) while this one is worked on: each warp
+//      pushes and deposits 32 particles that sit CH/32 places apart in the
+//      list (in a cell-sorted list that puts the lanes of a warp in
+//      different cells, so their current updates do not collide), and a
+//      coalesced store writes the chunk back,
 //   4. flushes the J tile once into 64-bit accumulators in global memory; a
 //      finalize pass folds the periodic guards and rounds each cell once to
 //      FP32, and
