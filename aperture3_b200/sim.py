@@ -467,6 +467,8 @@ class SimData:
                 src = (src.to(torch.int64) & 0xFFFFFFFF)
                 src = torch.where(src >= 2 ** 31, src - 2 ** 32, src).to(torch.int32)
             self.particles[name][:n].copy_(src)
+        # the copies wait on the caller's stream, the update runs on its own
+        torch.cuda.current_stream().synchronize()
         self.number = n
         self.particles_modified()
 
@@ -475,6 +477,7 @@ class SimData:
             if key in fields:
                 for c in range(3):
                     getattr(self, key)[c].copy_(fields[key][c])
+        torch.cuda.current_stream().synchronize()
 
     def particles_modified(self, number: Optional[int] = None):
         if number is not None:

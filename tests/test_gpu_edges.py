@@ -146,3 +146,32 @@ def test_sort_by_cell_around_its_tiles(n, order, half):
     got = {k: v[first:end] for k, v in pr.data.particles_host().items()}
     for k, _ in oracle.PTC_FIELDS:
         assert_bits(got[k], pr.p[k][:n_ref], f"sorted {k}")
+
+
+def test_update_waits_for_the_state_it_was_given():
+    """The state's tensors are still being written on the caller's stream when
+    the first update is called (a 0.1 s kernel in front of them): the update
+    sees all of them."""
+    import torch
+    from aperture3_b200 import SimData, SimEnvironment, ic, ptc_updater
+    params, fields, ptc = ic.box2d(seed=3, N=64, ppc=8, device=torch.device("cuda", 0))
+    n = ptc["x1"].numel()
+    got = []
+    for cycles in (0, int(2e8)):
+        env = SimEnvironment(params)
+        data = SimData(env, capacity=2 * n)
+        env.set_compaction(2)
+        torch.cuda.synchronize()
+        if cycles:
+            torch.cuda._sleep(cycles)
+        data.set_fields_device(fields)
+        data.set_particles_device({k: v.clone() for k, v in ptc.items()})
+        for step in range(2):
+            ptc_updater(env).update_particles(data, params.delta_t, step)
+        torch.cuda.synchronize()
+        a, b = data.slot_range()
+        got.append({k: v[a:b].clone() for k, v in data.particles.items()})
+        env.close()
+    assert int((got[1]["cell"] != -1).sum()) == n
+    for k in got[0]:
+        assert torch.equal(got[0][k], got[1][k]), k
