@@ -175,3 +175,25 @@ def test_update_waits_for_the_state_it_was_given():
     assert int((got[1]["cell"] != -1).sum()) == n
     for k in got[0]:
         assert torch.equal(got[0][k], got[1][k]), k
+
+
+@pytest.mark.parametrize("N,tile", [((63, 48), (16, 16)), ((37, 29), (8, 8)), ((97, 50), (32, 16))])
+@pytest.mark.parametrize("field_load", ["tma", "plain"])
+def test_2d_deposit_of_offsets_outside_the_cell(N, tile, field_load):
+    """Particles that their caller placed up to half a cell outside their cell
+    (and at -0.0, 1 and next to both) deposit the clamped weights of any
+    offset, at every node and face of their range. Free streaming, so that the
+    deposit alone is compared; the second step starts from moved offsets."""
+    n = 5000
+    params, m, rng, f = _state(N, n, 17, amp=0.0, tile=tile)
+    p = random_particles(m, n, rng, gamma_max=50.0)
+    one = np.float32(1)
+    sides = np.array([-0.45, -0.2, -1e-3, -1e-8, -0.0, 0.0, 0.5, 0.9, 1.0,
+                      np.nextafter(one, one * 2), 1.001, 1.3, 1.45], np.float32)
+    for k in ("x1", "x2"):
+        p[k][:] = sides[rng.integers(0, len(sides), n)]
+    pr = Pair(params, f, p, row_align=4 if field_load == "tma" else 1)
+    for step in range(2):
+        pr.both_update_particles(step)
+        pr.check_particles()
+        pr.check_current(J_TOL, rho=True)
