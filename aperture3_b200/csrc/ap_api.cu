@@ -188,10 +188,12 @@ int check_status(Ctx *c) {
   return AP_OK;
 }
 
-// The 2D work-item list of the current tiles and particle capacity.
+// The 2D work-item list of the current tiles and particle capacity, with room
+// for the items of every chunk length: the chunk can change while the list
+// stays (n particles in ntiles tiles make at most n / kMinChunk + ntiles).
 int alloc_items(Ctx *c) {
   if (c->mk.dim != 2) return AP_OK;
-  const size_t need = c->order_cap / (size_t)chunk_of(*c) + (size_t)c->tiles.ntiles + 2;
+  const size_t need = c->order_cap / (size_t)kMinChunk + (size_t)c->tiles.ntiles + 2;
   if (c->items_cap >= need) return AP_OK;
   cudaFree(c->items);
   c->items = nullptr;
@@ -312,7 +314,7 @@ AP_API int ap_ctx_create(const ap_mesh *mesh, const ap_params *params, ap_ctx **
             cudaMalloc(&c->tile_start[1], sizeof(uint32_t) * (nt + 1)) == cudaSuccess &&
             cudaMalloc(&c->diag_dev, sizeof(double) * 16) == cudaSuccess &&
             cudaMalloc(&c->fx_used, sizeof(FixedFmt)) == cudaSuccess &&
-            cudaMalloc(&c->n_max, 3 * sizeof(uint32_t)) == cudaSuccess &&
+            cudaMalloc(&c->n_max, 4 * sizeof(uint32_t)) == cudaSuccess &&
             cudaMalloc(&c->wmax, sizeof(float)) == cudaSuccess &&
             cudaMallocHost(&c->diag_host, sizeof(double) * 16) == cudaSuccess;
   if (!ok) {
@@ -322,7 +324,7 @@ AP_API int ap_ctx_create(const ap_mesh *mesh, const ap_params *params, ap_ctx **
   cudaMemset(c->diag_dev, 0xFF, sizeof(double) * 16);  // NaN: nothing recorded yet
   std::memset(c->status_host, 0, sizeof(DevStatus));
   cudaMemset(c->fx_used, 0, sizeof(FixedFmt));
-  cudaMemset(c->n_max, 0, 3 * sizeof(uint32_t));
+  cudaMemset(c->n_max, 0, 4 * sizeof(uint32_t));
   cudaMemset(c->wmax, 0, sizeof(float));
   *out = c;
   return AP_OK;

@@ -627,9 +627,9 @@ AP_API int ap_batch_autotune(ap_batch *b, const double *dt, const uint32_t *step
                         (c->mk.red[1] + cand[k][1] - 1) / cand[k][1] >= 3;
       if (fits) {
         ok[b->tune_class[r]] = true;
+        b->runs[r]->params.chunk = cand[k][2];
         st = ap_set_tile_shape(static_cast<ap_ctx *>(b->runs[r]), cand[k][0], cand[k][1]);
         if (st != AP_OK) break;
-        b->runs[r]->params.chunk = cand[k][2];
       }
     }
     // the first step after a shape change includes the order rebuild: time
@@ -657,9 +657,12 @@ AP_API int ap_batch_autotune(ap_batch *b, const double *dt, const uint32_t *step
       const int k = best_k[b->tune_class[r]];
       int tx = 0, ty = 0;
       ap_get_tile_shape(static_cast<ap_ctx *>(b->runs[r]), &tx, &ty);
-      if (tx != cand[k][0] || ty != cand[k][1])
-        st = ap_set_tile_shape(static_cast<ap_ctx *>(b->runs[r]), cand[k][0], cand[k][1]);
+      // a changed chunk rebuilds the order too: its work items are whole chunks
+      const bool same = tx == cand[k][0] && ty == cand[k][1] &&
+                        b->runs[r]->params.chunk == cand[k][2];
       b->runs[r]->params.chunk = cand[k][2];
+      if (!same)
+        st = ap_set_tile_shape(static_cast<ap_ctx *>(b->runs[r]), cand[k][0], cand[k][1]);
     }
   if (steps_used) *steps_used = used;
   return st;

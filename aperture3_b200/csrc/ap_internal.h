@@ -98,7 +98,9 @@ struct PushDepositParams {
   // work items: item k is list entries [items[k].y, items[k].y + item_len) of
   // tile items[k].x
   const uint2 *items;
-  const uint32_t *n_items;  // [0] their number, [1] item_len, a multiple of the chunk
+  // [0] their number, [1] item_len, a multiple of the chunk, [2] items that
+  // found no room in the list (never, by its size: reported as a tile fault)
+  const uint32_t *n_items;
   // per staged chunk of the tile lists, its direction counts (10 each):
   // chunk k of tile t is entry tile_start[t] / CH + t + k (null: not kept)
   uint32_t *chunk_count;
@@ -247,7 +249,7 @@ struct Ctx {
   size_t acc_comp = 0;
   size_t acc_offset = 0;        // of acc in the control block
   FixedFmt *fx_used = nullptr;  // device: format of the last deposit
-  uint32_t *n_max = nullptr;    // device: largest tile population, number of work items, item length
+  uint32_t *n_max = nullptr;    // device: largest tile population, then PushDepositParams::n_items
   float *wmax = nullptr;        // device: max |weight| over the bound particles
   bool scale_valid = false;
 
@@ -439,12 +441,13 @@ cudaError_t launch_ls_inject(Ctx &c, int inj, float p1, float w, uint64_t seed, 
 
 MeshK make_meshk(const ap_mesh &m);
 
-// Particles staged per chunk by the 2D push / deposit of this context: 1024
-// for log-spherical grids, else the configured 256, 1024 or 2048, or 512.
+// Particles staged per chunk by the 2D push / deposit of this context: 256
+// for log-spherical grids, else the configured 512, 1024 or 2048, or 256.
+constexpr int kMinChunk = 256;
 inline int chunk_of(const Ctx &c) {
-  if (c.coord == 1) return 256;
+  if (c.coord == 1) return kMinChunk;
   const int ch = c.params.chunk;
-  return (ch == 512 || ch == 1024 || ch == 2048) ? ch : 256;
+  return (ch == 512 || ch == 1024 || ch == 2048) ? ch : kMinChunk;
 }
 
 // The update of one context in three parts (ap_api.cu): prepare (zeroing,

@@ -308,7 +308,10 @@ __device__ __forceinline__ void push_deposit_tiles(const PushDepositParams &P0,
     const int lg = max(4, bits_of(*P.n_max));
     const FixedFmt fx = fixed_format(lg, 63 - 2 * lg, P.qmax * *P.wmax);
     const float fscale = ldexpf(1.0f, fx.S);
-    if (k == 0 && tid == 0) *P.fx_used = fx;
+    if (k == 0 && tid == 0) {
+      *P.fx_used = fx;
+      if (n_items[2]) atomicAdd(&P.status->tile_faults, (unsigned long long)n_items[2]);
+    }
 
     const int tix = t % P.t.ntx, tiy = t / P.t.ntx;
     const int x0 = g0 + tix * TX, y0 = g1 + tiy * TY;

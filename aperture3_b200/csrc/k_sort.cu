@@ -397,7 +397,7 @@ __global__ void k_tile_keys(MeshK m, TilesK T, uint32_t *cell, size_t base, size
 // start array that stands already.
 // The same pass lists the push / deposit's work items: a tile of n particles
 // gives ceil(n / item_len) of them, their number in n_max[1], item_len in
-// n_max[2].
+// n_max[2], those past the list's end in n_max[3].
 enum ScanSource { kCounts, kPop, kStarts };
 
 struct ItemOut {
@@ -481,6 +481,7 @@ __global__ void __launch_bounds__(kScanThreads)
       n_max[0] = mx;
       n_max[1] = min(icarry, I.cap);
       n_max[2] = I.len;
+      n_max[3] = icarry - min(icarry, I.cap);
     }
   }
 }

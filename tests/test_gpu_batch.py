@@ -22,12 +22,13 @@ def _specs(seed, nruns):
              int(rng.integers(2, 9)), seed * 1000 + r) for r in range(nruns)]
 
 
-def _make(spec, data_interval=2, spare=1, compact=0, tile=(0, 0)):
+def _make(spec, data_interval=2, spare=1, compact=0, tile=(0, 0), chunk=0, weight=None):
     N0, N1, ppc, s = spec
     n = N0 * N1 * ppc
     params = make_params((N0, N1), periodic=(True, True), capacity=spare * n,
                          data_interval=data_interval, tile=tile)
     params.delta_t = float(np.float32(0.45 / max(N0, N1)))
+    params.chunk = chunk
     rng = np.random.default_rng(s)
     m = mesh_2d(N0, N1)
     f = random_fields(m, rng, amp=0.3)
@@ -35,6 +36,8 @@ def _make(spec, data_interval=2, spare=1, compact=0, tile=(0, 0)):
         for c in range(3):
             oracle.send_guard_cells(m, f[key][c], (1, 1, 0))
     p = random_particles(m, n, rng, gamma_max=100.0)
+    if weight is not None:
+        p["weight"][:] = weight
     env = SimEnvironment(params)
     data = SimData(env, capacity=spare * n)
     data.set_fields(f)
@@ -108,6 +111,39 @@ def test_batch_autotune_then_steps():
     shapes = batch.tile_shapes()
     assert all(s in ((16, 16), (32, 16), (16, 8), (8, 8), (4, 4)) for s in shapes)
     _compare(alone, batched, tol=1e-6)
+    _close(batch, alone, batched)
+
+
+@pytest.mark.parametrize("chunk", [1024, 2048])
+def test_batch_autotune_of_runs_with_long_chunks(chunk):
+    """Runs created with 1024- or 2048-particle chunks and enough particles
+    that the candidates' shorter chunks cut the tile lists into more work items
+    than the run's own chunk would: no particle may be left out. The weights
+    are too small for the currents to reach the fields' last bits, so every
+    member and field must equal the untuned run's, in its slot."""
+    specs = [(256, 256, 16, 77)]
+    alone = [_make(s, weight=1e-20) for s in specs]
+    batched = [_make(s, weight=1e-20, chunk=chunk) for s in specs]
+    batch = Batch([d for _, d in batched])
+    used = batch.autotune(0)
+    batch.sync()
+    for step in range(used, used + 3):
+        batch.update_particles(step)
+        batch.update_fields(step)
+        batch.sync()
+    for step in range(used + 3):
+        _step_alone(alone, step)
+    for (_, da), (_, db) in zip(alone, batched):
+        pa, pb = da.particles_host(), db.particles_host()
+        for k in ("x1", "x2", "x3", "p1", "p2", "p3", "E", "cell", "flag", "weight", "id"):
+            assert_bits(pb[k], pa[k], f"particles.{k}")
+        fa, fb = da.fields_host(), db.fields_host()
+        for key in ("E", "B"):
+            for c in range(3):
+                assert_bits(fb[key][c], fa[key][c], f"{key}{c + 1}")
+        order, start = db.tile_order()
+        assert np.array_equal(np.sort(order), np.arange(len(pb["id"])))
+        assert start[-1] == len(pb["id"])
     _close(batch, alone, batched)
 
 
