@@ -686,13 +686,15 @@ __global__ void __launch_bounds__(kLineThreads)
 // Rows that fit shared memory twice: up to 28000 cells in one launch for all
 // rows and passes. 8192 cells, one pass of E3, J1 and two charge densities:
 // 9 launches of 1.6 us before, 2 here.
-bool line_smooth_fits(const Ctx &c) { return c.mesh.dims[0] <= 28000; }
+constexpr int kLineCells = 28000;
+bool line_smooth_fits(const Ctx &c) { return c.mesh.dims[0] <= kLineCells; }
 
 static cudaError_t launch_line_rows(Ctx &c, const LineRows &R, int rows, int passes) {
   const size_t smem = 2 * sizeof(float) * (size_t)c.mesh.dims[0];
-  if (smem > 48 * 1024) {
+  if (smem > 48 * 1024) {  // the longest row's, the same from every context and thread
     cudaError_t e = cudaFuncSetAttribute(k_line_smooth,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+                                         cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)(2 * sizeof(float) * kLineCells));
     if (e != cudaSuccess) return e;
   }
   const int b = !c.params.periodic[0];

@@ -188,9 +188,18 @@ struct TileGeom {
   static constexpr size_t stage1_bytes() {
     return stage_bytes() > raw_bytes() ? stage_bytes() : raw_bytes();
   }
-  static size_t smem_bytes(int nrho, bool ls = false) {
+  static constexpr size_t smem_bytes(int nrho, bool ls = false) {
     return HDR + rec_bytes() + stage0_bytes() + stage1_bytes() + 8 * (3 + nrho) * JSZ +
            (ls ? 4 * JSZ : 0) + order_bytes();
+  }
+  // The limit belongs to the kernel on its device, not to a context or a
+  // launch: every caller sets the same one, which holds any number of species
+  // (of the 227 KB a block may have, less the batch's parameters).
+  template <class Kernel>
+  static cudaError_t allow_smem(Kernel *kern) {
+    constexpr size_t most = smem_bytes(AP_MAX_SPECIES, true);
+    static_assert(most + sizeof(PushDepositParams) <= 227 * 1024, "shared memory of a block");
+    return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
   }
 };
 
@@ -1249,8 +1258,7 @@ cudaError_t launch_2d_tiles(Ctx &c, const PushDepositParams &P) {
   auto run = [&](auto kern) -> cudaError_t {
     // blocks per SM of the variant, asked for when the context's variant changes
     if (c.pd_kern != reinterpret_cast<const void *>(kern) || c.pd_smem != smem) {
-      cudaError_t err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             (int)smem);
+      cudaError_t err = G::allow_smem(kern);
       if (err != cudaSuccess) return err;
       int per_sm = 0;
       err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kThreads2D, smem);
@@ -1367,8 +1375,7 @@ cudaError_t launch_batch_tiles(cudaStream_t stream, int num_sms, bool tma, bool 
   const size_t smem = G::smem_bytes(do_rho ? max_species : 0);
   k_batch_bases<<<1, 32, 0, stream>>>(runs, nruns, base, queue);
   auto run = [&](auto kern) -> cudaError_t {
-    cudaError_t err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           (int)smem);
+    cudaError_t err = G::allow_smem(kern);
     if (err != cudaSuccess) return err;
     int per_sm = 0;
     err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kThreads2D, smem);

@@ -197,3 +197,87 @@ def test_2d_deposit_of_offsets_outside_the_cell(N, tile, field_load):
         pr.both_update_particles(step)
         pr.check_particles()
         pr.check_current(J_TOL, rho=True)
+
+
+@pytest.mark.parametrize("kind", ["box", "logsph"])
+def test_contexts_of_different_species_counts_take_turns(kind):
+    """Contexts with three and with two charge densities share their kernel
+    but not the shared memory of a launch: each runs again after the other."""
+    import torch
+    from aperture3_b200 import SimData, SimEnvironment, ic, ptc_updater
+    from aperture3_b200.sim import ptc_updater_logsph
+    dev = torch.device("cuda", 0)
+    runs = []
+    for species in (3, 2):
+        if kind == "logsph":
+            params, fields, ptc = ic.logsph(seed=3, N=64, ppc=8, device=dev)
+        else:
+            params, fields, ptc = ic.box2d(seed=3, N=64, ppc=8, device=dev)
+        params.num_species, params.data_interval, params.tile_size = species, 1, (16, 16, 0)
+        env = SimEnvironment(params)
+        data = SimData(env, capacity=ptc["x1"].numel())
+        data.set_fields_device(fields)
+        data.set_particles_device(ptc)
+        runs.append((env, data))
+    cls = ptc_updater_logsph if kind == "logsph" else ptc_updater
+    for step in range(3):
+        for env, data in runs:
+            cls(env).update_particles(data, env.params.delta_t, step)
+    (_, a), (_, b) = runs
+    for k in a.particles:
+        assert torch.equal(a.particles[k], b.particles[k]), k
+    for s in range(2):
+        assert torch.equal(a.Rho[s], b.Rho[s])
+    assert not a.Rho[2].any()
+    for env, _ in runs:
+        env.close()
+
+
+def test_smoothing_of_rows_of_different_lengths_from_two_threads():
+    """The 1D gap lab's rows in shared memory: two threads with rows of
+    different lengths smooth at the same time, and get what they get alone."""
+    import threading
+    import torch
+    from aperture3_b200 import SimData, SimEnvironment, SimParams
+    from aperture3_b200.sim import ptc_updater_1dgap
+
+    def make(N):
+        p = SimParams(N=(N, 1, 1), guard=(2, 0, 0), lower=(0.0, 0.0, 0.0), size=(1.0, 1.0, 1.0),
+                      delta_t=0.5 / N, q_e=1.0, num_species=2, current_smoothing=2,
+                      periodic_boundary=(False, False, False), max_ptc_number=1, B0=0.7,
+                      coord_system="1dgap")
+        env = SimEnvironment(p)
+        data = SimData(env, capacity=1)
+        g = torch.Generator().manual_seed(N)
+        data.E[0].copy_(torch.randn(data.E[0].shape, generator=g))
+        torch.cuda.synchronize()
+        return env, data
+
+    def smooth(env, data, times):
+        for _ in range(times):
+            ptc_updater_1dgap(env).update_particles(data, env.params.delta_t, 0)
+
+    sizes = (7000, 25000)
+    want = []
+    for N in sizes:
+        env, data = make(N)
+        smooth(env, data, 1)
+        want.append(data.E[2].clone())
+        env.close()
+    runs, failed = [make(N) for N in sizes], []
+
+    def body(env, data):
+        try:
+            smooth(env, data, 200)
+        except Exception as e:  # noqa: BLE001 (reported below)
+            failed.append(e)
+
+    threads = [threading.Thread(target=body, args=r) for r in runs]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not failed
+    for (env, data), w in zip(runs, want):
+        assert torch.equal(data.E[2], w)
+        env.close()
