@@ -8,6 +8,7 @@ goes through libaperture_b200.so; device memory comes from torch.
 """
 from __future__ import annotations
 
+import contextlib
 import ctypes as C
 import dataclasses
 from typing import Callable, Dict, List, Optional, Sequence
@@ -402,6 +403,20 @@ class SimData:
         check(self.env._lib.ap_bind_photons(self.env.ctx, C.byref(ph), int(number),
                                             self.photon_capacity), "ap_bind_photons")
 
+    @contextlib.contextmanager
+    def _writing(self):
+        """Around copies into the state's arrays: they run on the caller's
+        stream of the arrays' device, the updates on the context's own. Waits
+        for the updates queued so far, which still use the arrays, and then
+        for the copies, which the next update reads. While the caller's stream
+        is captured the order is the capture's and nothing waits."""
+        capturing = torch.cuda.is_current_stream_capturing()
+        if not capturing:
+            self.stats()  # waits for the context's stream, reports no fault
+        yield
+        if not capturing:
+            torch.cuda.current_stream(self.env.device).synchronize()
+
     # -- photons ---------------------------------------------------------
     @property
     def photon_number(self) -> int:
@@ -424,11 +439,12 @@ class SimData:
         n = len(host["x1"])
         if n > self.photon_capacity:
             raise _lib.ApError(5, "set_photons")
-        for name, dt in PH_FIELDS:
-            a = np.ascontiguousarray(host[name])
-            t = torch.from_numpy(a.view(np.int32) if dt == torch.int32 else
-                                 (a.view(np.int64) if dt == torch.int64 else a))
-            self.photons[name][:n].copy_(t)
+        with self._writing():
+            for name, dt in PH_FIELDS:
+                a = np.ascontiguousarray(host[name])
+                t = torch.from_numpy(a.view(np.int32) if dt == torch.int32 else
+                                     (a.view(np.int64) if dt == torch.int64 else a))
+                self.photons[name][:n].copy_(t)
         self._bind_photons(n)
 
     def photons_host(self) -> Dict[str, np.ndarray]:
@@ -447,11 +463,12 @@ class SimData:
         n = len(host["x1"])
         if n > self.capacity:
             raise _lib.ApError(5, "set_particles")
-        for name, dt in PTC_FIELDS:
-            a = np.ascontiguousarray(host[name])
-            t = torch.from_numpy(a.view(np.int32) if dt == torch.int32 else
-                                 (a.view(np.int64) if dt == torch.int64 else a))
-            self.particles[name][:n].copy_(t)
+        with self._writing():
+            for name, dt in PTC_FIELDS:
+                a = np.ascontiguousarray(host[name])
+                t = torch.from_numpy(a.view(np.int32) if dt == torch.int32 else
+                                     (a.view(np.int64) if dt == torch.int64 else a))
+                self.particles[name][:n].copy_(t)
         self.number = n
         self.particles_modified()
 
@@ -461,23 +478,22 @@ class SimData:
         n = ptc["x1"].numel()
         if n > self.capacity:
             raise _lib.ApError(5, "set_particles_device")
-        for name, dt in PTC_FIELDS:
-            src = ptc[name]
-            if dt == torch.int32 and src.dtype != torch.int32:
-                src = (src.to(torch.int64) & 0xFFFFFFFF)
-                src = torch.where(src >= 2 ** 31, src - 2 ** 32, src).to(torch.int32)
-            self.particles[name][:n].copy_(src)
-        # the copies wait on the caller's stream, the update runs on its own
-        torch.cuda.current_stream().synchronize()
+        with self._writing():
+            for name, dt in PTC_FIELDS:
+                src = ptc[name]
+                if dt == torch.int32 and src.dtype != torch.int32:
+                    src = (src.to(torch.int64) & 0xFFFFFFFF)
+                    src = torch.where(src >= 2 ** 31, src - 2 ** 32, src).to(torch.int32)
+                self.particles[name][:n].copy_(src)
         self.number = n
         self.particles_modified()
 
     def set_fields_device(self, fields: Dict[str, List[torch.Tensor]]):
-        for key in ("E", "B", "Ebg", "Bbg", "J"):
-            if key in fields:
-                for c in range(3):
-                    getattr(self, key)[c].copy_(fields[key][c])
-        torch.cuda.current_stream().synchronize()
+        with self._writing():
+            for key in ("E", "B", "Ebg", "Bbg", "J"):
+                if key in fields:
+                    for c in range(3):
+                        getattr(self, key)[c].copy_(fields[key][c])
 
     def particles_modified(self, number: Optional[int] = None):
         if number is not None:
@@ -569,13 +585,15 @@ class SimData:
         }
 
     def set_fields(self, host):
-        for key in ("E", "B", "Ebg", "Bbg", "J"):
-            if key in host:
-                for c in range(3):
-                    getattr(self, key)[c].copy_(torch.from_numpy(np.ascontiguousarray(host[key][c])))
-        if "Rho" in host:
-            for s, a in enumerate(host["Rho"]):
-                self.Rho[s].copy_(torch.from_numpy(np.ascontiguousarray(a)))
+        with self._writing():
+            for key in ("E", "B", "Ebg", "Bbg", "J"):
+                if key in host:
+                    for c in range(3):
+                        getattr(self, key)[c].copy_(
+                            torch.from_numpy(np.ascontiguousarray(host[key][c])))
+            if "Rho" in host:
+                for s, a in enumerate(host["Rho"]):
+                    self.Rho[s].copy_(torch.from_numpy(np.ascontiguousarray(a)))
 
 
 def _wrap_device_ptr(ptr: int, n: int) -> torch.Tensor:

@@ -281,3 +281,38 @@ def test_smoothing_of_rows_of_different_lengths_from_two_threads():
     for (env, data), w in zip(runs, want):
         assert torch.equal(data.E[2], w)
         env.close()
+
+
+@pytest.mark.parametrize("from_host", [False, True])
+def test_setters_wait_for_queued_updates(from_host):
+    """Particles and fields are replaced while pipelined updates of the old
+    ones are still queued: the new state is as in a context that had none."""
+    import torch
+    from aperture3_b200 import SimData, SimEnvironment, ic, ptc_updater
+    dev = torch.device("cuda", 0)
+    params, fields, ptc = ic.box2d(seed=3, N=256, ppc=32, device=dev)
+    _, fields2, ptc2 = ic.box2d(seed=4, N=256, ppc=32, device=dev)
+    n = ptc["x1"].numel()
+    got = []
+    for queued in (0, 30):
+        env = SimEnvironment(params)
+        data = SimData(env, capacity=n)
+        data.set_fields_device(fields)
+        data.set_particles_device(ptc)
+        env.set_sync(False)
+        pusher = ptc_updater(env)
+        for step in range(queued):
+            pusher.update_particles(data, params.delta_t, step)
+        if from_host:
+            host = ic.to_numpy_ptc(ptc2)
+            data.set_fields({k: [f.cpu().numpy() for f in v] for k, v in fields2.items()})
+            data.set_particles(host)
+        else:
+            data.set_fields_device(fields2)
+            data.set_particles_device(ptc2)
+        pusher.update_particles(data, params.delta_t, 0)
+        env.sync()
+        got.append([t.clone() for t in (*data.particles.values(), *data.J, *data.E, *data.B)])
+        env.close()
+    for a, b in zip(*got):
+        assert torch.equal(a, b)

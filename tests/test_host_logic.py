@@ -1,11 +1,15 @@
 """Host-side logic of the Python mirror that needs no device: the mesh
 built as Grid::init does, charges and masses as setup_env does, the
 parameter file reader, and the seeded initial conditions."""
+import types
+
 import numpy as np
+import pytest
+import torch
 
 import oracle
-from aperture3_b200 import ic
-from aperture3_b200.sim import SimEnvironment, SimParams
+from aperture3_b200 import ic, sim
+from aperture3_b200.sim import SimData, SimEnvironment, SimParams
 
 
 def test_mesh_matches_grid_init():
@@ -46,3 +50,47 @@ def test_box1d_initial_state():
     assert ptc["x1"].numel() == 4096
     assert abs(float(ptc["p1"].std()) - 0.1) < 0.01
     assert float(fields["B"][0].min()) == 1.0
+
+
+@pytest.mark.parametrize("capturing", [False, True])
+def test_setters_wait_on_the_arrays_device(monkeypatch, capturing):
+    """A setter waits for the context's queued work, copies, and waits for the
+    stream of the arrays' device (another device may be current); under
+    capture it only copies."""
+    log = []
+
+    class Stream:
+        def __init__(self, device):
+            self.device = device
+
+        def synchronize(self):
+            log.append(("copies", self.device))
+
+    class Tensor(torch.Tensor):
+        def copy_(self, src, *a):
+            log.append("copy")
+            return super().copy_(src)
+
+    monkeypatch.setattr(torch.cuda, "current_stream", lambda device=None: Stream(device))
+    monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: capturing)
+    data = SimData.__new__(SimData)
+    data.env = types.SimpleNamespace(device=torch.device("cuda", 1))
+    data.capacity = 4
+    data.stats = lambda: log.append("updates")
+    data.particles_modified = lambda: log.append("modified")
+    zeros = lambda dt=torch.float32: torch.zeros(4, dtype=dt).as_subclass(Tensor)  # noqa: E731
+    data.particles = {name: zeros(dt) for name, dt in sim.PTC_FIELDS}
+    for key in ("E", "B", "Ebg", "Bbg", "J"):
+        setattr(data, key, [zeros() for _ in range(3)])
+    waits = (["updates"], [("copies", data.env.device)]) if not capturing else ([], [])
+    ptc = {name: torch.ones(3, dtype=dt) for name, dt in sim.PTC_FIELDS}
+    host = {k: v.numpy() for k, v in ptc.items()}
+    n = len(sim.PTC_FIELDS)
+    for call, copies, after in ((lambda: data.set_particles_device(ptc), n, ["modified"]),
+                                (lambda: data.set_particles(host), n, ["modified"]),
+                                (lambda: data.set_fields_device({"E": [torch.ones(4)] * 3}), 3, []),
+                                (lambda: data.set_fields({"E": [np.ones(4, np.float32)] * 3}), 3,
+                                 [])):
+        log.clear()
+        call()
+        assert log == waits[0] + ["copy"] * copies + waits[1] + after
