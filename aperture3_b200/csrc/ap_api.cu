@@ -55,7 +55,8 @@ cudaError_t alloc_control(Ctx &c) {
   c.queue = reinterpret_cast<uint32_t *>(b + sizeof(DevStatus));
   c.dir_count = reinterpret_cast<uint32_t *>(b + kControlHead);
   c.acc = reinterpret_cast<unsigned long long *>(b + c.acc_offset);
-  return cudaMemset(b, 0, c.acc_offset);
+  // on the context's stream: the default stream's work is not ordered with it
+  return cudaMemsetAsync(b, 0, c.acc_offset, c.stream);
 }
 
 cudaError_t clear_control(Ctx &c, int ncomp) {
@@ -321,11 +322,11 @@ AP_API int ap_ctx_create(const ap_mesh *mesh, const ap_params *params, ap_ctx **
     ap_ctx_destroy(c);
     return AP_ERR_NOMEM;
   }
-  cudaMemset(c->diag_dev, 0xFF, sizeof(double) * 16);  // NaN: nothing recorded yet
+  cudaMemsetAsync(c->diag_dev, 0xFF, sizeof(double) * 16, c->stream);  // NaN: nothing recorded yet
   std::memset(c->status_host, 0, sizeof(DevStatus));
-  cudaMemset(c->fx_used, 0, sizeof(FixedFmt));
-  cudaMemset(c->n_max, 0, 4 * sizeof(uint32_t));
-  cudaMemset(c->wmax, 0, sizeof(float));
+  cudaMemsetAsync(c->fx_used, 0, sizeof(FixedFmt), c->stream);
+  cudaMemsetAsync(c->n_max, 0, 4 * sizeof(uint32_t), c->stream);
+  cudaMemsetAsync(c->wmax, 0, sizeof(float), c->stream);
   *out = c;
   return AP_OK;
 }
@@ -414,7 +415,7 @@ AP_API int ap_bind_fields(ap_ctx *c, const ap_fields *f) {
   if (!c->tmp_j) {
     size_t pitch = sizeof(float) * (size_t)m.dims[0];
     AP_TRY(cudaMalloc(&c->tmp_j, pitch * (size_t)m.dims[1] * m.dims[2]));
-    AP_TRY(cudaMemset(c->tmp_j, 0, pitch * (size_t)m.dims[1] * m.dims[2]));
+    AP_TRY(cudaMemsetAsync(c->tmp_j, 0, pitch * (size_t)m.dims[1] * m.dims[2], c->stream));
     c->tmp_pitch = m.dims[0];
   }
   return AP_OK;

@@ -382,7 +382,8 @@ int ensure_pair_scratch(Ctx &c) {
   if (cudaMalloc(&c.pair_chunks, sizeof(uint32_t) * (2 * cap + 8)) != cudaSuccess)
     return AP_ERR_NOMEM;
   // the mark pass adds into the counts, the scan resets them
-  if (cudaMemset(c.pair_chunks, 0, sizeof(uint32_t) * (2 * cap + 8)) != cudaSuccess)
+  if (cudaMemsetAsync(c.pair_chunks, 0, sizeof(uint32_t) * (2 * cap + 8), c.stream) !=
+      cudaSuccess)
     return AP_ERR_CUDA;
   c.pair_cap_chunks = cap;
   return AP_OK;

@@ -316,3 +316,32 @@ def test_setters_wait_for_queued_updates(from_host):
         env.close()
     for a, b in zip(*got):
         assert torch.equal(a, b)
+
+
+def test_a_new_tile_shape_is_ordered_with_the_updates():
+    """The buffers of a new tile shape are cleared in the updates' order, not
+    in that of the default stream, whose earlier work (a kernel of some 10 ms
+    here) ends while the updates run."""
+    import torch
+    from aperture3_b200 import SimData, SimEnvironment, ic, ptc_updater
+    dev = torch.device("cuda", 0)
+    params, fields, ptc = ic.box2d(seed=3, N=128, ppc=16, device=dev)
+    got = []
+    for cycles in (0, int(2e7)):
+        env = SimEnvironment(params)
+        data = SimData(env, capacity=ptc["x1"].numel())
+        data.set_fields_device(fields)
+        data.set_particles_device(ptc)
+        env.set_sync(False)
+        torch.cuda.synchronize()
+        if cycles:
+            torch.cuda._sleep(cycles)
+        env.set_tile_shape(8, 8)
+        for step in range(400):
+            ptc_updater(env).update_particles(data, params.delta_t, step)
+        env.sync()
+        torch.cuda.synchronize()
+        got.append([t.clone() for t in (*data.particles.values(), *data.J)])
+        env.close()
+    for a, b in zip(*got):
+        assert torch.equal(a, b)
