@@ -442,13 +442,10 @@ cudaError_t launch_ls_inject(Ctx &c, int inj, float p1, float w, uint64_t seed, 
 MeshK make_meshk(const ap_mesh &m);
 
 // Particles staged per chunk by the 2D push / deposit of this context: 256
-// for log-spherical grids, else the configured 512, 1024 or 2048, or 256.
+// for log-spherical grids, else the configured 512, 1024 or 2048, or 256, or
+// the next one that leaves room for a second CTA on the SM (k_push_deposit.cu).
 constexpr int kMinChunk = 256;
-inline int chunk_of(const Ctx &c) {
-  if (c.coord == 1) return kMinChunk;
-  const int ch = c.params.chunk;
-  return (ch == 512 || ch == 1024 || ch == 2048) ? ch : kMinChunk;
-}
+int chunk_of(const Ctx &c);
 
 // The update of one context in three parts (ap_api.cu): prepare (zeroing,
 // tile-order rebuild, kernel parameters), the push / deposit launch, and

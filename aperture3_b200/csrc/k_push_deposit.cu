@@ -1332,6 +1332,47 @@ cudaError_t launch_fixed_scale(Ctx &c) {
   return cudaGetLastError();
 }
 
+namespace {
+
+template <int TX, int TY>
+size_t cta_bytes(int chunk, int nrho) {
+  const size_t dyn = chunk == 2048   ? TileGeom<TX, TY, 2048>::smem_bytes(nrho)
+                     : chunk == 1024 ? TileGeom<TX, TY, 1024>::smem_bytes(nrho)
+                     : chunk == 512  ? TileGeom<TX, TY, 512>::smem_bytes(nrho)
+                                     : TileGeom<TX, TY, 256>::smem_bytes(nrho);
+  return dyn + sizeof(PushDepositParams);  // a batch's copy of the parameters
+}
+
+}  // namespace
+
+// The configured chunk while the current and charge tiles of all species leave
+// room for a second CTA on the SM (228 KB, 1 KB reserved per CTA), else the
+// next shorter one that does (512 for 256, whose two buffers take more). Alone
+// on its SM a CTA has nothing to hide its barriers behind: 512^2 cells x 32
+// particles with charges, us per update, one CTA and by this rule (and before
+// the field records, which take the room, two CTAs): 16x16/2048 with 2 species
+// 985, 574 (764); 16x8/2048 with 8 species 1049, 604 (797); 32x16/1024 with 6
+// 1007, 722 (788); 32x16/256 with 8 927, 726 (764); 32x16/2048 with 2 966, 674
+// (1056, one CTA then too). Three CTAs in place of four, and two in place of
+// three, cost less than the records give: 16x16/256 with 3 species 523 (600),
+// 32x16/256 with 2 611 (712), 16x16/1024 with 3 636 (672).
+int chunk_of(const Ctx &c) {
+  if (c.coord == 1) return kMinChunk;
+  const int want = c.params.chunk == 512 || c.params.chunk == 1024 || c.params.chunk == 2048
+                       ? c.params.chunk : kMinChunk;
+  const int tx = c.tiles.tx, ty = c.tiles.ty, ns = c.params.num_species;
+  const int tries[3] = {want, 1024, 512};
+  for (int ch : tries) {
+    if (ch > want && ch != 512) continue;
+    const size_t bytes = tx == 32 ? cta_bytes<32, 16>(ch, ns)
+                         : ty == 16 ? cta_bytes<16, 16>(ch, ns)
+                         : tx == 16 ? cta_bytes<16, 8>(ch, ns)
+                         : tx == 8 ? cta_bytes<8, 8>(ch, ns) : cta_bytes<4, 4>(ch, ns);
+    if (2 * (bytes + 1024) <= 228 * 1024) return ch;
+  }
+  return want;
+}
+
 cudaError_t launch_push_deposit_2d(Ctx &c, const PushDepositParams &P) {
   const int tx = P.t.tx, ty = P.t.ty;
   if (tx == 16 && ty == 16) return launch_2d_chunk<16, 16>(c, P);

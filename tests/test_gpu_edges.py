@@ -345,3 +345,23 @@ def test_a_new_tile_shape_is_ordered_with_the_updates():
         env.close()
     for a, b in zip(*got):
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("tile,chunk,species", [((16, 16), 2048, 1), ((16, 16), 2048, 2),
+                                                ((16, 8), 2048, 8), ((8, 8), 2048, 2),
+                                                ((4, 4), 2048, 3), ((32, 16), 0, 2),
+                                                ((32, 16), 0, 8), ((32, 16), 1024, 6),
+                                                ((32, 16), 2048, 2), ((16, 16), 1024, 4)])
+def test_2d_chunks_and_species_on_both_sides_of_the_shared_memory_rule(tile, chunk, species):
+    """Tiles, chunks and species counts whose CTA leaves room for a second one
+    on the SM, and some that take a shorter chunk instead; tiles of one to
+    several work items."""
+    n = 60000
+    params, m, rng, f = _state((97, 50), n, 23, tile=tile)
+    params.chunk, params.num_species = chunk, species
+    p = random_particles(m, n, rng, gamma_max=5.0, species=range(species))
+    pr = Pair(params, f, p)
+    for step in range(2):
+        pr.both_update_particles(step)
+        pr.check_particles()
+        pr.check_current(J_TOL, rho=True)
