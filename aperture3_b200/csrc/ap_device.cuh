@@ -29,7 +29,7 @@ __device__ __forceinline__ float cic(float dx) {
 // the three nodes c-1, c, c+1; for an offset in [0, 1] at most two of them
 // carry a nonzero weight, and which two is decided exactly:
 //  - stagger 1 (node at t + 1): nodes c-1 and c; node c+1 sits at distance
-//    (c + 2) - (c + rel) >= 1.
+//    (c + 2) - (c + rel) >= 1 (for an offset above 1: nodes c, c+1).
 //  - stagger 0 (node at t + 0.5): nodes c-1, c when c + rel < c + 0.5,
 //    otherwise c, c+1; the skipped node is at distance >= 1.
 // Skipping a node whose weight is exactly zero leaves the accumulated sum
@@ -39,36 +39,53 @@ __device__ __forceinline__ float cic(float dx) {
 // exact: the distances are f, 1 - f, |0.5 - f| and so on, so the weights are
 // 1 - f and f (stagger 1), and 0.5 -+ f or 1.5 - f, f - 0.5 (stagger 0), the
 // same bits as the reference's fl(1 - |node - xc|) in a third of the
-// instructions. Offsets outside [0, 1], NaNs and cells further out take the
-// expressions themselves.
+// instructions (weights_inside). Offsets outside [0, 1], NaNs and cells
+// further out take the expressions themselves (weights_any).
 struct Weights1D {
   int base0;       // first node for stagger 0 (c-1 or c)
+  int base1;       // and for stagger 1 (c-1; c for an offset above 1)
   float w0[2];     // stagger-0 weights of nodes base0, base0 + 1
-  float w1[2];     // stagger-1 weights of nodes c-1, c
+  float w1[2];     // stagger-1 weights of nodes base1, base1 + 1
 };
 
-__device__ __forceinline__ Weights1D weights_1d(float rel, int c) {
+constexpr int kExactCells = 1 << 22;
+
+__device__ __forceinline__ Weights1D weights_inside(float rel, int c) {
+  Weights1D W;
+  const float fc = (float)c;
+  const float f = (rel + fc) - fc;
+  const bool low = f < 0.5f;
+  W.base0 = low ? c - 1 : c;
+  W.base1 = c - 1;
+  W.w1[0] = 1.0f - f;
+  W.w1[1] = f;
+  W.w0[0] = (low ? 0.5f : 1.5f) - f;
+  W.w0[1] = f + (low ? 0.5f : -0.5f);
+  return W;
+}
+
+__device__ __forceinline__ Weights1D weights_any(float rel, int c) {
   Weights1D W;
   const float fc = (float)c;
   const float xc = rel + fc;
-  const float f = xc - fc;
-  // one test of the bits: f is in [0, 1] and no NaN
-  if (__float_as_uint(f) <= __float_as_uint(1.0f) && c < (1 << 22)) {
-    const bool low = f < 0.5f;
-    W.base0 = low ? c - 1 : c;
-    W.w1[0] = 1.0f - f;
-    W.w1[1] = f;
-    W.w0[0] = (low ? 0.5f : 1.5f) - f;
-    W.w0[1] = f + (low ? 0.5f : -0.5f);
-  } else {
-    W.base0 = xc < fc + 0.5f ? c - 1 : c;
-    const float fb = (float)W.base0;
-    W.w1[0] = cic(((float)(c - 1) + 1.0f) - xc);
-    W.w1[1] = cic((fc + 1.0f) - xc);
-    W.w0[0] = cic((fb + 0.5f) - xc);
-    W.w0[1] = cic(((float)(W.base0 + 1) + 0.5f) - xc);
-  }
+  W.base0 = xc < fc + 0.5f ? c - 1 : c;
+  W.base1 = xc > fc + 1.0f ? c : c - 1;
+  const float f0 = (float)W.base0, f1 = (float)W.base1;
+  W.w1[0] = cic((f1 + 1.0f) - xc);
+  W.w1[1] = cic(((float)(W.base1 + 1) + 1.0f) - xc);
+  W.w0[0] = cic((f0 + 0.5f) - xc);
+  W.w0[1] = cic(((float)(W.base0 + 1) + 0.5f) - xc);
   return W;
+}
+
+// Whether offsets are in [0, 1] (one test of the bits; -0 and NaNs are not).
+__device__ __forceinline__ bool offsets_inside(float a, float b) {
+  return max(__float_as_uint(a), __float_as_uint(b)) <= __float_as_uint(1.0f);
+}
+
+__device__ __forceinline__ Weights1D weights_1d(float rel, int c) {
+  return offsets_inside(rel, rel) && c < kExactCells ? weights_inside(rel, c)
+                                                     : weights_any(rel, c);
 }
 
 // Quotients by one divisor b, each the correctly rounded a / b: y is the

@@ -35,6 +35,8 @@
 #include <cuda.h>
 #include <cuda_runtime.h>
 
+#include <type_traits>
+
 #include "ap_device.cuh"
 #include "ap_internal.h"
 
@@ -212,6 +214,8 @@ __device__ __forceinline__ int spos(int e) { return e + (e >> 5); }
 constexpr uint8_t kWritePos = 1;  // x1, x2, x3, cell
 constexpr uint8_t kWriteMom = 2;  // p1, p2, p3, E
 constexpr uint8_t kWriteFlag = 4; // flag (log-spherical outflow)
+// Direction and mode of an element left to the second walk of its chunk.
+constexpr uint8_t kLeft = 0xff;
 
 // Shared-memory copy of one run's parameters (batched launches only).
 template <bool kMulti>
@@ -311,6 +315,7 @@ __device__ __forceinline__ void push_deposit_tiles(const PushDepositParams &P0,
     uint32_t *s_ord = reinterpret_cast<uint32_t *>(s_dv + (kLS ? G::JSZ : 0));
     const int dims0 = P.m.dims[0], dims1 = P.m.dims[1];
     const int g0 = P.m.guard[0], g1 = P.m.guard[1];
+    const bool exact_grid = dims0 <= kExactCells && dims1 <= kExactCells;
     const int nacc = ncomp * G::JSZ;
 
     // fixed-point format of this update, from the largest tile population
@@ -448,10 +453,11 @@ __device__ __forceinline__ void push_deposit_tiles(const PushDepositParams &P0,
       uint32_t *s_flag = reinterpret_cast<uint32_t *>(stc + 8 * SP);
       uint32_t *s_idx = reinterpret_cast<uint32_t *>(stc + 9 * SP);
       uint8_t *s_dm = reinterpret_cast<uint8_t *>(stc + 10 * SP);  // direction, mode << 4
-      // 3b. push + deposit: lane l of warp w takes element l*CH/32 + w*PER_THREAD + k
-      for (int k = 0; k < PER_THREAD; ++k) {
-        const int e = lane * (CH / 32) + warp * PER_THREAD + k;
-        if (e >= nch) continue;
+      // 3b. push + deposit of one element. kAny: with the expressions for any
+      // offset; without, for offsets in [0, 1] on grids of at most kExactCells
+      // a side.
+      auto particle = [&](auto any, const int e) {
+        constexpr bool kAny = decltype(any)::value;
         const int s = spos(e);
         const uint32_t c = s_cell[s];
         const uint32_t flag = s_flag[s];
@@ -482,8 +488,10 @@ __device__ __forceinline__ void push_deposit_tiles(const PushDepositParams &P0,
           if constexpr (kLS) r_push = expf(mesh_pos(P.m.lower[0], P.m.delta[0], c1, g0, x1));
           if (em) {
             const float qm = P.qm[sp];
-            const Weights1D Wx = weights_1d(x1, c1);
-            const Weights1D Wy = weights_1d(x2, c2);
+            const Weights1D Wx = kLS ? weights_1d(x1, c1)
+                                 : kAny ? weights_any(x1, c1) : weights_inside(x1, c1);
+            const Weights1D Wy = kLS ? weights_1d(x2, c2)
+                                 : kAny ? weights_any(x2, c2) : weights_inside(x2, c2);
             // each component: its four nodes in the reference's order, times
             // the x weight, then the y weight, added up from zero
             float fe[6];
@@ -498,8 +506,8 @@ __device__ __forceinline__ void push_deposit_tiles(const PushDepositParams &P0,
               acc += b.y;
               return acc * qm;
             };
-            const int i0 = Wx.base0 - (x0 - 1), i1 = lx;
-            const int j0 = (Wy.base0 - ys) * G::RX, j1 = ly * G::RX;
+            const int i0 = Wx.base0 - (x0 - 1), i1 = Wx.base1 - (x0 - 1);
+            const int j0 = (Wy.base0 - ys) * G::RX, j1 = (Wy.base1 - ys) * G::RX;
             {
               const float4 r0 = sEB[j1 + i0], r1 = sEB[j1 + G::RX + i0];
               fe[0] = comp(make_float2(r0.x, r0.y), make_float2(r1.x, r1.y), Wx.w0, Wy.w1);
@@ -617,11 +625,7 @@ __device__ __forceinline__ void push_deposit_tiles(const PushDepositParams &P0,
               const Acc32 R{sJhi + (3 + sp) * G::JSZ, sJlo + (3 + sp) * G::JSZ};
               const bool rho = kRho && P.do_rho && sp < P.num_species;
               const int o = (ly + jb + 2) * G::JX + (lx + ib + 2);
-              // one test of the bits; the other branch out of the way of this
-              // one (512^2 x 32: 441 us per update without it, 445 so, 448 with
-              // the branches laid out as they come)
-              if (__builtin_expect(max(__float_as_uint(x1), __float_as_uint(x2)) <=
-                                       __float_as_uint(1.0f), 1)) {
+              if constexpr (!kAny) {
                 // old weights 1 - x, x on the nodes -1, 0; new ones 1 - nx, nx
                 // on -1 + dc, dc; the window starts at -2 for dc = -1, else -1
                 float sx0[3], sx1[3], sy0[3], sy1[3];
@@ -810,8 +814,33 @@ __device__ __forceinline__ void push_deposit_tiles(const PushDepositParams &P0,
         const unsigned stay = __ballot_sync(act, dir == 4u);
         if (lane == __ffs(act) - 1) atomicAdd(&s_cnt[4], (uint32_t)__popc(stay));
         if (dir != 4u) atomicAdd(&s_cnt[dir], 1u);
+      };
+      // lane l of warp w takes element l*CH/32 + w*PER_THREAD + k. Offsets
+      // outside [0, 1] (particles their caller placed so, once: the move leaves
+      // offsets inside) are left to a second walk: in branches of the first one
+      // their expressions cost every particle (512^2 x 32: 441 us per update
+      // without them, 445 with those of the deposit in a branch, 450 with those
+      // of the weights too, 444 so).
+      bool rest = false;
+      for (int k = 0; k < PER_THREAD; ++k) {
+        const int e = lane * (CH / 32) + warp * PER_THREAD + k;
+        if (e >= nch) continue;
+        if (kLS || (exact_grid && offsets_inside(s_x1[spos(e)], s_x2[spos(e)]))) {
+          particle(std::false_type{}, e);
+        } else {
+          s_dm[spos(e)] = kLeft;
+          rest = true;
+        }
       }
-      __syncthreads();
+      if constexpr (kLS) {
+        __syncthreads();
+      } else if (__syncthreads_or(rest)) {
+        for (int k = 0; k < PER_THREAD; ++k) {
+          const int e = lane * (CH / 32) + warp * PER_THREAD + k;
+          if (e < nch && s_dm[spos(e)] == kLeft) particle(std::true_type{}, e);
+        }
+        __syncthreads();
+      }
       // direction counts of this chunk, for the one-pass order update
       if (P.chunk_count && tid < 10) {
         const uint32_t v = s_cnt[tid];
@@ -922,9 +951,9 @@ constexpr int kItems1D = 8;
 constexpr int kChunk1D = kThreads1D * kItems1D;  // 2048 particles
 constexpr int kWin1D = 6000;                     // cell-components per window
 
-__device__ __forceinline__ float interp_1d_global(const FieldArr &f, const Weights1D &W, int c1,
+__device__ __forceinline__ float interp_1d_global(const FieldArr &f, const Weights1D &W,
                                                   int stag) {
-  const int b = stag ? c1 - 1 : W.base0;
+  const int b = stag ? W.base1 : W.base0;
   const float w0 = stag ? W.w1[0] : W.w0[0];
   const float w1 = stag ? W.w1[1] : W.w0[1];
   float acc = 0.0f;
@@ -1112,7 +1141,7 @@ __device__ __forceinline__ void push_deposit_1d_chunk(const PushDepositParams &P
       const Weights1D W = weights_1d(x1, c1);
       float fe[6];
 #pragma unroll
-      for (int q = 0; q < 6; ++q) fe[q] = interp_1d_global(P.F[q], W, c1, stag_x(q)) * qm;
+      for (int q = 0; q < 6; ++q) fe[q] = interp_1d_global(P.F[q], W, stag_x(q)) * qm;
       vay_push_v(p1, p2, p3, gamma, fe[0], fe[1], fe[2], fe[3], fe[4], fe[5], v1, v2, v3);
       P.p.p1[idx] = p1;
       P.p.p2[idx] = p2;

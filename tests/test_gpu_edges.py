@@ -365,3 +365,22 @@ def test_2d_chunks_and_species_on_both_sides_of_the_shared_memory_rule(tile, chu
         pr.both_update_particles(step)
         pr.check_particles()
         pr.check_current(J_TOL, rho=True)
+
+
+@pytest.mark.parametrize("N", [(63, 48), (512,)])
+def test_fields_at_offsets_outside_the_cell(N):
+    """Particles placed up to half a cell outside their cell are pushed by the
+    fields there, bit for bit: above 1 the third node of a component counts."""
+    n = 5000
+    params, m, rng, f = _state(N, n, 19, amp=0.05)
+    p = random_particles(m, n, rng, gamma_max=2.0)
+    one = np.float32(1)
+    sides = np.array([-0.45, -0.2, -1e-3, -1e-8, -0.0, 0.0, 0.5, 0.9, 1.0,
+                      np.nextafter(one, one * 2), 1.001, 1.3, 1.45], np.float32)
+    for k in ("x1", "x2")[:m.dimension]:
+        p[k][:] = sides[rng.integers(0, len(sides), n)]
+    pr = Pair(params, f, p)
+    for step in range(2):
+        pr.both_update_particles(step)
+        pr.check_particles()
+        pr.check_current(J_TOL, rho=True)
