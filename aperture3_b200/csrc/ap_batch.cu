@@ -4,11 +4,11 @@
 // stream and without host synchronisation: each run's zeroing (and tile
 // order rebuild when needed), ONE persistent push / deposit launch per
 // group of runs that share a tile shape, chunk and field-load path (CTAs
-// draw (run, tile) items from one queue over all the group's tiles, so
-// small runs fill the GPU together), then each run's order update and
-// current finalize. The per-run kernel parameters and tensor maps go to
-// the device as an array of RunDesc through a double-buffered pinned
-// staging area.
+// draw work items -- tile lists or parts of them -- from one queue over all
+// the group's runs, so small runs fill the GPU together), then each run's
+// order update and current finalize. The per-run kernel parameters and
+// tensor maps go to the device as an array of RunDesc through a
+// double-buffered pinned staging area.
 #include <cuda_runtime.h>
 
 #include <algorithm>

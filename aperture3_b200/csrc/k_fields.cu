@@ -162,7 +162,10 @@ __global__ void k_divs(Geo G, Arr e1, Arr e2, Arr b1, Arr b2, Arr e01, Arr e02, 
 // update_fields of a small grid (the optional half step of E, then B, E and
 // the divergences) in one launch: one cluster of eight CTAs, a cluster barrier
 // between the stages in place of a launch. Small CTAs, so that they find room
-// beside another run's push.
+// beside another run's push. The line lies at two cells per thread: three
+// launches take 12.3 us up to 65536 cells (latency), the cluster 6.2 us for 1024
+// cells, 9.1 (1D) and 10.3 (64^2) for 4096, 12.3 for 72^2, 14.3 for 8192 and 22.5
+// for 16384.
 constexpr int kSmallThreads = 256;
 constexpr int kSmallCtas = 8;
 constexpr int kSmallCells = 2 * kSmallThreads * kSmallCtas;

@@ -916,8 +916,9 @@ __global__ void __launch_bounds__(kThreads2D, MINB)
   push_deposit_tiles<TX, TY, CH, kTMA, kRho, kLS, false>(P, maps.m, nullptr, nullptr, 0, P.queue);
 }
 
-// Many independent Cartesian runs in one persistent launch: CTAs take
-// (run, tile) work items from one queue over all runs' tiles.
+// Many independent Cartesian runs in one persistent launch: CTAs take work
+// items (a tile's list of one run, or a part of it) from one queue over all
+// runs' items.
 template <int TX, int TY, int CH, int MINB, bool kTMA, bool kRho>
 __global__ void __launch_bounds__(kThreads2D, MINB)
     k_push_deposit_2d_batch(const RunDesc *__restrict__ runs, const uint32_t *__restrict__ base,

@@ -603,9 +603,11 @@ TileTopo topo_of(const Ctx &c) {
                   c.params.periodic[1]};
 }
 
-// Work items of the next push: about three per resident CTA (four per SM), so
-// that neither a grid of few tiles nor a few crowded tiles leave the rest of
-// the chip idle at the end; a tile of at most one item's length stays whole.
+// Work items of the next push: about three per resident CTA of the variants
+// with four CTAs per SM, so that neither a grid of few tiles nor a few crowded
+// tiles leave the rest of the chip idle at the end; variants with two or three
+// get the same lengths, four to six items per CTA. A tile of at most one item's
+// length stays whole.
 // An item costs its field tile, a cleared and a flushed current tile, about
 // 2 us beside the 3 - 6 us of a 256-particle chunk.
 ItemOut item_out(Ctx &c) {
