@@ -384,3 +384,23 @@ def test_fields_at_offsets_outside_the_cell(N):
         pr.both_update_particles(step)
         pr.check_particles()
         pr.check_current(J_TOL, rho=True)
+
+
+def test_logsph_push_at_offsets_outside_the_cell():
+    """Log-spherical particles placed up to 0.4 cells outside their cell (away
+    from the axis): pushed as near the FP64 oracle as the FP32 oracle is, with
+    the bounds of the ordinary step."""
+    from oracle import logsph as ls
+    from test_gpu_logsph import LsCase, _check_against_f64
+    case = LsCase((128, 64), 40000, 3)
+    rng = np.random.default_rng(29)
+    row = case.p["cell"].astype(np.int64) // case.m.dims[0] - case.m.guard[1]
+    far = (row >= 3) & (row < 64 - 3)
+    sides = np.array([-0.4, -0.2, -1e-3, 0.0, 0.5, 1.0, 1.001, 1.2, 1.4], np.float32)
+    for k in ("x1", "x2"):
+        case.p[k][far] = sides[rng.integers(0, len(sides), case.n)][far]
+    case.p64 = ls.to_f64(case.p)
+    case.data.set_particles(case.p)
+    case.step_particles(0)
+    _check_against_f64(case, "offsets outside the cell")
+    case.close()
